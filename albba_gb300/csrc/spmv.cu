@@ -19,23 +19,24 @@
 // never read: a lane stops at its row's length, so the fma chain is the
 // reference's, bit for bit.
 //
-// Rows longer than kSpLong entries (the hubs of a power-law graph) keep an
-// empty SELL row: in a slice a hub's lane waits on one group of x gathers at
-// a time and holds its warp -- and the whole launch -- for tens of
-// milliseconds. They are copied in CSR order to a separate list (longest
-// first, each row padded to 8 entries so that a lane reads its row in
-// aligned 32-byte column and 64-byte value blocks) and summed lane per row
-// by k_spmv_long, which keeps two blocks of x gathers in flight ahead of the
-// fma chain. The chain itself stays sequential -- its order is what makes y
-// bit-identical -- and a dependent fp64 fma costs about 90 cycles on GB300
-// (the fp64 pipe takes as long for one active lane as for 32), so the launch
-// can end no sooner than the longest row's length x that latency; lane per
-// row keeps every other row's chains, 32 per warp instruction, off the fp64
-// pipe's critical path. The long rows run on a side stream beside the slices.
+// Rows longer than kSpLong entries keep an empty SELL row: in a slice such a
+// row's lane waits on one group of x gathers at a time and holds its warp for
+// milliseconds. They are kept in a list of their own, longest first. The
+// chain of fused multiply-adds is what makes y bit-identical, and a dependent
+// fp64 fma costs about 115 cycles on GB300 (for one active lane as for 32), so
+// the list is summed in two ways: shorter ones lane per row (k_spmv_long: 32 chains side by side), the hubs
+// CTA per row with the chain's steps found 256 at a time as integers
+// (k_spmv_hub, chain.cuh), so that the longest row's chain no longer sets the
+// launch's length. Each runs on a stream of its own beside the slices. R-MAT
+// scale 22, edge factor 16, signed values: 9.47 ms with every long row lane
+// per row, 2.1 ms now; with positive values 0.84 ms.
 #include <algorithm>
+#include <cmath>
 #include <cstring>
+#include <functional>
 #include <vector>
 
+#include "chain.cuh"
 #include "graph.h"
 #include "ingest.h"
 #include "scan.cuh"
@@ -43,30 +44,33 @@
 struct alb_sellmat {
     int device = 0;
     cudaStream_t stream = nullptr;
-    cudaStream_t side = nullptr;  // the long rows run beside the slices
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr, fork = nullptr, join = nullptr;
+    cudaStream_t side = nullptr, side2 = nullptr;  // hubs, long rows: beside the slices
+    cudaEvent_t ev0 = nullptr, ev1 = nullptr, fork = nullptr, join = nullptr, join2 = nullptr;
     int64_t n = 0, nnz = 0, nslices = 0, stored = 0;
     int32_t sigma = 0;
+    int32_t num_sms = 0;
+    int32_t wslices = 1;           // slices per sort window where windows are whole slices, else 1
     int32_t *perm = nullptr;       // position -> row
     int32_t *deg = nullptr;        // row length by position
     int64_t *slice_off = nullptr;  // first entry of each slice (multiple of 128)
     int32_t *col = nullptr;        // 4-interleaved column ids
     double *val = nullptr;         // values, same layout
     double *dx = nullptr, *dy = nullptr;  // staging for host vectors
-    int64_t nlong = 0;             // rows longer than kSpLong, summed by a warp each
+    int64_t nlong = 0;             // rows longer than kSpLong
+    int64_t nhub = 0;              // the first of them, CTA per row (hub_threshold)
     int32_t *lrow = nullptr;       // their row ids, longest first
-    int64_t *lptr = nullptr;       // first entry of each in lcol / lval (multiple of 8)
+    int64_t *lptr = nullptr;       // first entries in lcol / lval: of each hub (a multiple of
+                                   // 8), then of each slice of 32 other long rows (of 128)
     int32_t *llen = nullptr;       // their lengths
-    int32_t *lcol = nullptr;       // their entries in CSR order, each row padded to 8
+    int32_t *lcol = nullptr;       // their entries: hubs row by row, the others interleaved
     double *lval = nullptr;
-    int32_t max_long = 0;          // the longest row's length
 };
 
 namespace alb {
 namespace {
 
 constexpr int kSpC = 32;
-constexpr int32_t kSpLong = 512;  // longer rows are summed by a warp each
+constexpr int32_t kSpLong = 256;  // longer rows leave the slices
 
 unsigned blocks_for(int64_t work, int block) {
     int64_t g = (work + block - 1) / block;
@@ -125,23 +129,31 @@ __global__ void k_sp_fill(int64_t n, int64_t npad, const int32_t *perm, const in
     }
 }
 
-// Warp per slice, lane per row. The next group's columns and values are
-// requested before this group's x gathers are used, so each lane keeps the
-// stream and the gathers in flight together.
-// 512 threads a block (32 K registers): such a block does not fit on an SM
-// beside a solo long-row CTA (k_spmv_long<true>), which keeps the slices off
-// the longest chains' SMs.
-constexpr int kSpBlock = 512;
+// Warp per slice, lane per row. While a group's four fmas run (a dependent
+// fma takes about 115 cycles), the next group's x gathers and the columns and
+// values after them are in flight.
+// Slices are taken rank by rank: the first (longest rows) of every sort
+// window, then every window's second, and so on. In index order a grid stride
+// that is a multiple of the slices per window hands one warp the longest
+// slice of window after window: at R-MAT scale 22 that warp set the kernel's
+// 1.66 ms. Small blocks: a matrix of a few hundred slices then spreads over
+// the SMs, whose fp64 pipe takes 16 cycles per warp and fma.
+constexpr int kSpBlock = 128;
 
-__global__ void __launch_bounds__(kSpBlock) k_spmv(int64_t n, int64_t nslices, const int32_t *perm,
-                                              const int32_t *deg, const int64_t *slice_off,
-                                              const int32_t *col, const double *val,
-                                              const double *x, double *y) {
+__global__ void __launch_bounds__(kSpBlock)
+    k_spmv(int64_t n, int64_t nslices, int32_t wslices, const int32_t *perm, const int32_t *deg,
+           const int64_t *slice_off, const int32_t *col, const double *val, const double *x,
+           double *y) {
     const int lane = threadIdx.x & 31;
-    const int64_t w0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const uint32_t w0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
     const uint64_t pol = l2_evict_first();
-    for (int64_t s = w0; s < nslices; s += nw) {
+    const uint32_t nwin = (uint32_t)((nslices + wslices - 1) / wslices);
+    const uint32_t total = nwin * (uint32_t)wslices;  // below 2^26 + sigma / 32
+    for (uint32_t i = w0; i < total; i += nw) {
+        const uint32_t rank = i / nwin;
+        const int64_t s = (int64_t)(i - rank * nwin) * wslices + rank;
+        if (s >= nslices) continue;  // the last window may be short
         const int64_t p = s * kSpC + lane;
         const int32_t dr = p < n ? __ldg(deg + p) : 0;
         const bool mine = p < n && dr <= kSpLong;  // long rows: k_spmv_long
@@ -153,143 +165,326 @@ __global__ void __launch_bounds__(kSpBlock) k_spmv(int64_t n, int64_t nslices, c
         double acc = 0.0;
         int4 c = make_int4(0, 0, 0, 0);
         double2 va = make_double2(0.0, 0.0), vb = va;
+        double xv[4];
+        // a group's gathers, c being its columns (padding is not followed)
+        auto gather = [&](const int4 &q, int32_t left, double (&v)[4]) {
+            v[0] = left > 0 ? __ldg(x + q.x) : 0.0;
+            v[1] = left > 1 ? __ldg(x + q.y) : 0.0;
+            v[2] = left > 2 ? __ldg(x + q.z) : 0.0;
+            v[3] = left > 3 ? __ldg(x + q.w) : 0.0;
+        };
         if (ng > 0) {
             c = ld_stream(cp, pol);
             va = __ldcs(vp);
             vb = __ldcs(vp + 1);
         }
+        gather(c, d, xv);
+        if (ng > 1) c = ld_stream(cp + kSpC, pol);
         for (int32_t g = 0; g < ng; g++) {
-            int4 cn = c;
+            const int32_t left = d - 4 * g;
             double2 van = va, vbn = vb;
+            double xn[4];
+            gather(c, left - 4, xn);
             if (g + 1 < ng) {
-                cn = ld_stream(cp + (int64_t)(g + 1) * kSpC, pol);
                 van = __ldcs(vp + (int64_t)(g + 1) * 2 * kSpC);
                 vbn = __ldcs(vp + (int64_t)(g + 1) * 2 * kSpC + 1);
             }
-            const int32_t left = d - 4 * g;
-            const double x0 = __ldg(x + c.x);
-            const double x1 = left > 1 ? __ldg(x + c.y) : 0.0;
-            const double x2 = left > 2 ? __ldg(x + c.z) : 0.0;
-            const double x3 = left > 3 ? __ldg(x + c.w) : 0.0;
-            acc = fma(va.x, x0, acc);
-            if (left > 1) acc = fma(va.y, x1, acc);
-            if (left > 2) acc = fma(vb.x, x2, acc);
-            if (left > 3) acc = fma(vb.y, x3, acc);
-            c = cn;
+            if (g + 2 < ng) c = ld_stream(cp + (int64_t)(g + 2) * kSpC, pol);
+            acc = fma(va.x, xv[0], acc);
+            if (left > 1) acc = fma(va.y, xv[1], acc);
+            if (left > 2) acc = fma(vb.x, xv[2], acc);
+            if (left > 3) acc = fma(vb.y, xv[3], acc);
             va = van;
             vb = vbn;
+#pragma unroll
+            for (int k = 0; k < 4; k++) xv[k] = xn[k];
         }
         if (mine) y[__ldg(perm + p)] = acc;
     }
 }
 
-// Lane per long row (rows longest first). kSolo: the launch's longest rows,
-// one per CTA of 1024 threads of which one lane works: the CTA holds most of
-// its SM's registers until the row ends, so no slices block shares the SM
-// and its fp64 pipe with the chain that sets the SpMV's length (measured: a
-// slices kernel beside the longest chain slowed it from 8.0 to about 10 ms at
-// RMAT s22), and the chain waits on no other lane's gathers (a warp's
-// cp.async wait ends when its slowest lane's copies land). The other long
-// rows go 32 of similar length per warp.
-// Entries in blocks of kLb. Each lane streams its row through two
-// shared-memory rings filled by cp.async: column ids kLd blocks ahead of the
-// x gathers that need them, values and x (each gather 8 bytes) kLd blocks
-// ahead of the fmas. The group committed at step t carries block t's values
-// and gathers and block t + kLd's columns, so one wait gives both. With the
-// fma chain at about 90 cycles per entry, each load has kLd x kLb entries'
-// worth of chain time to land. Ring layout: lane-fastest, so that the 32
-// lanes' accesses fall in different banks.
+// Lane per long row, 32 rows of similar length per warp (longest first),
+// interleaved as in a slice. Bound: the longest row's chain, about 58 ns per
+// entry. Every load has to land within the chain time of the groups before
+// it: columns are requested 2 kLd groups of four entries ahead, values and x
+// gathers kLd groups (kLd x 4 fmas, near 2 us) ahead, all in registers. Rings
+// in shared memory (cp.async) left the SM's L1 too small to hold the gathers
+// in flight: 1.5 ms at R-MAT scale 22 instead of 0.7, and 6 ms with the
+// slices' gathers beside it.
 constexpr int kSpLongBlock = 32;  // one warp per CTA
-constexpr int kLb = 8;
-constexpr int kLd = 8;
+constexpr int kLb = 8;            // hub rows are padded to this many entries
+constexpr int kLd = 4;
 
-__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async8(void *dst, const void *src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-constexpr int kSoloThreads = 1024;
-constexpr int64_t kSoloRows = 8;  // rows on CTAs of their own
-
-template <bool kSolo>
-__global__ void __launch_bounds__(kSolo ? kSoloThreads : kSpLongBlock)
-    k_spmv_long(int64_t nlong, int64_t first, const int32_t *lrow, const int64_t *lptr,
-                const int32_t *llen, const int32_t *lcol, const double *lval, const double *x,
-                double *y) {
-    __shared__ double2 s_v[1][kLd][kLb / 2][32];
-    __shared__ double s_x[1][kLd][kLb][32];
-    __shared__ int4 s_c[1][kLd][kLb / 4][32];
-    // kSolo: warp 0 of CTA b takes row first + b on lane 0 (the other warps
-    // leave at once); otherwise warp w takes rows first + 32 w + lane
-    if (kSolo && threadIdx.x >= 32) return;
-    const int lane = threadIdx.x & 31, wib = 0;
-    const int64_t i = kSolo ? (lane == 0 ? first + blockIdx.x : nlong)
-                            : first + (int64_t)blockIdx.x * 32 + lane;
-    const int64_t b = i < nlong ? lptr[i] : 0;
-    const int64_t e = i < nlong ? b + llen[i] : 0;
-    const int64_t nblk = (e - b + kLb - 1) / kLb;
-    // values and x of block t (columns c); columns of block t + kLd
-    auto issue = [&](int64_t t, const int32_t (&c)[kLb]) {
-        const int slot = (int)(t % kLd);
-        if (t < nblk) {
-            const int64_t s0 = b + t * kLb;
-            const double2 *src = reinterpret_cast<const double2 *>(lval + s0);
-#pragma unroll
-            for (int h = 0; h < kLb / 2; h++) cp_async16(&s_v[wib][slot][h][lane], src + h);
-#pragma unroll
-            for (int k = 0; k < kLb; k++)
-                if (s0 + k < e) cp_async8(&s_x[wib][slot][k][lane], x + c[k]);
-        }
-        if (t + kLd < nblk) {
-            const int4 *src = reinterpret_cast<const int4 *>(lcol + b + (t + kLd) * kLb);
-#pragma unroll
-            for (int h = 0; h < kLb / 4; h++) cp_async16(&s_c[wib][slot][h][lane], src + h);
-        }
-        cp_async_commit();
+__global__ void __launch_bounds__(kSpLongBlock)
+    k_spmv_long(int64_t nrows, const int32_t *lrow, const int64_t *moff, const int32_t *llen,
+                const int32_t *lcol, const double *lval, const double *x, double *y) {
+    const int lane = threadIdx.x & 31;
+    const int64_t i = (int64_t)blockIdx.x * kSpC + lane;
+    const int32_t len = i < nrows ? llen[i] : 0;
+    const int32_t ng = (len + 3) >> 2;
+    const int64_t base = moff[blockIdx.x] + 4 * lane;
+    const int4 *cp = reinterpret_cast<const int4 *>(lcol + base);
+    const double2 *vp = reinterpret_cast<const double2 *>(lval + base);
+    int4 c[kLd];
+    double2 va[kLd], vb[kLd];
+    double xv[kLd][4];
+    // group g: its columns into c[j]; its values and gathers (padding points
+    // at x[0] and is not used)
+    auto cols = [&](int j, int32_t g) {
+        if (g < ng) c[j] = __ldcs(cp + (int64_t)g * kSpC);
     };
-    int32_t c[kLb];
-    for (int t = 0; t < kLd; t++) {
+    auto fetch = [&](int j, int32_t g) {
+        if (g >= ng) return;
+        va[j] = __ldcs(vp + (int64_t)g * 2 * kSpC);
+        vb[j] = __ldcs(vp + (int64_t)g * 2 * kSpC + 1);
+        xv[j][0] = __ldg(x + c[j].x);
+        xv[j][1] = __ldg(x + c[j].y);
+        xv[j][2] = __ldg(x + c[j].z);
+        xv[j][3] = __ldg(x + c[j].w);
+    };
 #pragma unroll
-        for (int k = 0; k < kLb; k++) c[k] = 0;
-        if (t < nblk) {
-            const int4 *q = reinterpret_cast<const int4 *>(lcol + b + (int64_t)t * kLb);
-            const int4 u = __ldcs(q), w = __ldcs(q + 1);
-            c[0] = u.x, c[1] = u.y, c[2] = u.z, c[3] = u.w;
-            c[4] = w.x, c[5] = w.y, c[6] = w.z, c[7] = w.w;
-        }
-        issue(t, c);
+    for (int j = 0; j < kLd; j++) cols(j, j);
+#pragma unroll
+    for (int j = 0; j < kLd; j++) {
+        fetch(j, j);
+        cols(j, kLd + j);
     }
     double acc = 0.0;
-    for (int64_t t = 0; t < nblk; t++) {
-        cp_async_wait<kLd - 1>();  // this lane's group t has landed
-        const int slot = (int)(t % kLd);
-        const int64_t rem = e - (b + t * kLb);
+    for (int32_t g0 = 0; g0 < ng; g0 += kLd) {
 #pragma unroll
-        for (int h = 0; h < kLb / 2; h++) {
-            const double2 v = s_v[wib][slot][h][lane];
-            if (2 * h < rem) acc = fma(v.x, s_x[wib][slot][2 * h][lane], acc);
-            if (2 * h + 1 < rem) acc = fma(v.y, s_x[wib][slot][2 * h + 1][lane], acc);
+        for (int j = 0; j < kLd; j++) {
+            const int32_t g = g0 + j, left = len - 4 * g;
+            if (left > 0) acc = fma(va[j].x, xv[j][0], acc);
+            if (left > 1) acc = fma(va[j].y, xv[j][1], acc);
+            if (left > 2) acc = fma(vb[j].x, xv[j][2], acc);
+            if (left > 3) acc = fma(vb[j].y, xv[j][3], acc);
+            fetch(j, g + kLd);
+            cols(j, g + 2 * kLd);
         }
-        // block t + kLd's columns (landed with group t), read out before the
-        // slot is refilled; the refill comes after the fmas in program order,
-        // so their shared loads have landed when the copies issue
-        const int4 u = s_c[wib][slot][0][lane], w = s_c[wib][slot][1][lane];
-        c[0] = u.x, c[1] = u.y, c[2] = u.z, c[3] = u.w;
-        c[4] = w.x, c[5] = w.y, c[6] = w.z, c[7] = w.w;
-        asm volatile("" ::"d"(acc), "r"(c[0]), "r"(c[7]) : "memory");
-        issue(t + kLd, c);
     }
-    cp_async_wait<0>();
-    if (i < nlong) y[lrow[i]] = acc;
+    if (i < nrows) y[lrow[i]] = acc;
+}
+
+// CTA per hub row, 256 entries a tile, the chain's steps as integer prefix
+// sums (chain.cuh). Warp 0 walks the chain. Warps 1 to 3 load: each takes
+// every third tile, keeps its columns six tiles and its values and x gathers
+// three tiles ahead in registers, and hands values, x and products over in
+// shared memory. Warps 4 to 6 scan the next tile for the exponent the
+// sum has now and its two neighbours. One block barrier a tile. Bound: warp
+// 0's latency on the longest row -- a look through a tile's prefixes, and for
+// each entry where the sum leaves its binade (a random walk of N signed terms
+// does so about 8 sqrt(N) times) one fma and another look; the sum mostly
+// moves between neighbouring binades, so the scans for them are at hand, and
+// warp 0 scans for any other exponent itself (the last two are kept). After a
+// step that leaves the sum small against its term, kRunSeq entries are done
+// by fma: there every second entry would end a run.
+constexpr int kTile = 256, kPer = kTile / 32;  // lane l: entries 8l .. 8l + 7
+constexpr int kHubFeed = 3, kHubScan = 3;      // warps that load, that scan
+constexpr int kHubThreads = 32 * (1 + kHubFeed + kHubScan);
+constexpr int kRunSeq = 8;
+
+struct HubTile {
+    double v[kPer][32], x[kPer][32];
+    int64_t h[kPer][32];  // the exact products (ChainTerm)
+    int16_t e[kPer][32];
+};
+
+// Tiles first, first + kHubFeed, ... of a row, one feeding warp.
+struct HubFeed {
+    const int32_t *lcol;
+    const double *lval, *x;
+    int64_t at, end;  // this lane's first entry of the tile held; the row's end
+    int32_t c[kPer];  // columns of the tile after the held one
+    double v[kPer], xv[kPer];
+
+    __device__ __forceinline__ void cols(int64_t e) {
+        if (e >= end) return;  // rows are padded to kPer: a lane's block is whole or absent
+        const int4 *q = reinterpret_cast<const int4 *>(lcol + e);
+        const int4 a = __ldcs(q), b = __ldcs(q + 1);
+        c[0] = a.x, c[1] = a.y, c[2] = a.z, c[3] = a.w;
+        c[4] = b.x, c[5] = b.y, c[6] = b.z, c[7] = b.w;
+    }
+    __device__ __forceinline__ void fetch() {
+        if (at >= end) return;
+        const double2 *q = reinterpret_cast<const double2 *>(lval + at);
+#pragma unroll
+        for (int h = 0; h < kPer / 2; h++) {
+            const double2 w = __ldcs(q + h);
+            v[2 * h] = w.x, v[2 * h + 1] = w.y;
+        }
+#pragma unroll
+        for (int k = 0; k < kPer; k++) xv[k] = __ldg(x + c[k]);
+    }
+    __device__ __forceinline__ void start(int64_t e) {
+        at = e;
+#pragma unroll
+        for (int k = 0; k < kPer; k++) c[k] = 0, v[k] = xv[k] = 0.0;
+        cols(at);
+        fetch();
+        cols(at + kHubFeed * kTile);
+    }
+    // the held tile goes to shared memory, the next one is requested
+    __device__ __forceinline__ void hand(HubTile &t) {
+        const int lane = threadIdx.x & 31;
+#pragma unroll
+        for (int k = 0; k < kPer; k++) {
+            t.v[k][lane] = v[k];
+            t.x[k][lane] = xv[k];
+            const bool in = at + k < end;  // an entry past the end adds nothing
+            const ChainTerm p = chain_term(in ? (uint64_t)__double_as_longlong(v[k]) : 0,
+                                           in ? (uint64_t)__double_as_longlong(xv[k]) : 0);
+            t.h[k][lane] = p.h;
+            t.e[k][lane] = (int16_t)p.e;
+        }
+        at += kHubFeed * kTile;
+        fetch();
+        cols(at + kHubFeed * kTile);
+    }
+};
+
+// Prefix sums of k over a tile, up to and with each entry, for one exponent.
+struct HubSums {
+    int64_t P[kPer][32];
+    uint8_t stop[32];  // each lane's entries that end a run: too large, or a tie
+};
+
+// One warp scans a tile for exponent E.
+__device__ __forceinline__ void hub_scan(const HubTile &T, int E, HubSums &out) {
+    const int lane = threadIdx.x & 31;
+    unsigned stop = 0;
+    int64_t q[kPer];
+#pragma unroll
+    for (int k = 0; k < kPer; k++) {
+        bool st;
+        q[k] = chain_round(T.h[k][lane], T.e[k][lane], E, st);
+        stop |= st ? 1u << k : 0u;
+    }
+#pragma unroll
+    for (int k = 1; k < kPer; k++) q[k] += q[k - 1];
+    const int64_t ex = warp_inclusive_scan(q[kPer - 1]) - q[kPer - 1];
+#pragma unroll
+    for (int k = 0; k < kPer; k++) out.P[k][lane] = q[k] + ex;
+    out.stop[lane] = (uint8_t)stop;
+}
+
+__global__ void __launch_bounds__(kHubThreads)
+    k_spmv_hub(const int32_t *lrow, const int64_t *lptr, const int32_t *llen, const int32_t *lcol,
+               const double *lval, const double *x, double *y) {
+    __shared__ HubTile s_t[3];
+    // by tile parity, exponents guess - 1 .. guess + 1; then warp 0's own two
+    __shared__ HubSums s_h[2 * kHubScan + 2];
+    // by tile parity: exponent of the sum after the tile; the tile's guess
+    __shared__ int s_E[2], s_guess[2];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int64_t len = llen[blockIdx.x];
+    const int64_t beg = lptr[blockIdx.x];
+    const int64_t ntile = (len + kTile - 1) / kTile;
+    HubFeed feed;
+    if (wib > 0 && wib <= kHubFeed) {
+        feed.lcol = lcol;
+        feed.lval = lval;
+        feed.x = x;
+        feed.end = beg + len;
+        feed.start(beg + (wib - 1) * kTile + kPer * lane);
+        if (wib <= 2) feed.hand(s_t[wib - 1]);
+    }
+    if (threadIdx.x == 0) s_E[0] = s_E[1] = s_guess[0] = s_guess[1] = -2;  // near no exponent
+    double acc = 0.0;
+    for (int64_t t = 0; t < ntile; t++) {
+        __syncthreads();  // tiles t and t + 1 and tile t's scans are in place
+        if (wib > kHubFeed) {
+            const int E = s_E[(t + 1) & 1];  // of the sum after tile t - 1
+            if (t + 1 < ntile && E > 0)
+                hub_scan(s_t[(t + 1) % 3], E + wib - kHubFeed - 2,
+                         s_h[((t + 1) & 1) * kHubScan + wib - kHubFeed - 1]);
+            if (wib == kHubFeed + 1 && lane == 0) s_guess[(t + 1) & 1] = E;
+            continue;
+        }
+        if (wib > 0) {
+            if ((t + 2) % kHubFeed == wib - 1 && t + 2 < ntile) feed.hand(s_t[(t + 2) % 3]);
+            continue;
+        }
+        const HubTile &T = s_t[t % 3];
+        const int guess = s_guess[t & 1];
+        const int cnt = (int)min((int64_t)kTile, len - t * kTile);
+        const unsigned here = cnt - kPer * lane >= kPer ? 0xFFu
+                              : cnt <= kPer * lane      ? 0u
+                                                        : (1u << (cnt - kPer * lane)) - 1u;
+        const int ahead = (int)(t & 1) * kHubScan + 1 - guess;  // + E: the prepared scan
+        int E0 = -1, E1 = -1, last = 0;  // exponents of warp 0's own two; the one used last
+        int ep = -4096;                  // biased exponent of the last product done by fma
+        int s = 0;                       // entries done
+        while (s < cnt) {
+            const uint64_t ab = (uint64_t)__double_as_longlong(acc);
+            const int E = (int)(ab >> 52) & 0x7FF;
+            int run = kRunSeq;
+            const bool ready = (unsigned)(E - guess + 1) < 3u;
+            // (a scan for an exponent that was not prepared pays only where
+            // the sum stands clear of its terms)
+            if (E > 0 && E < 0x7FF && (ready || E == E0 || E == E1 || E >= ep + 4)) {
+                int h = ahead + E;
+                if (!ready) {
+                    if (E != E0 && E != E1) {
+                        last = E0 < 0 ? 0 : E1 < 0 ? 1 : 1 - last;
+                        __syncwarp();
+                        hub_scan(T, E, s_h[2 * kHubScan + last]);
+                        __syncwarp();
+                        if (last) E1 = E;
+                        else E0 = E;
+                    }
+                    last = E == E0 ? 0 : 1;
+                    h = 2 * kHubScan + last;
+                }
+                const HubSums &H = s_h[h];
+                // A = base + P (acc > 0) or base - P (acc < 0), less 2^52 + 1 so
+                // that an entry's result is inside when its bits 52 and up are 0
+                const int64_t sg = (int64_t)ab >> 63;
+                const int64_t P0 = s > 0 ? H.P[(s - 1) & 7][(s - 1) >> 3] : 0;
+                const int64_t A0 = (int64_t)(ab & ((uint64_t)kChainOne - 1));
+                const int64_t base = A0 - 1 - sg - ((P0 ^ sg) - sg);
+                unsigned out = H.stop[lane];
+#pragma unroll
+                for (int k = 0; k < kPer; k++) {
+                    const int64_t w = (H.P[k][lane] ^ sg) + base;
+                    out |= (uint32_t)((uint64_t)w >> 32) >= 0x00100000u ? 1u << k : 0u;
+                }
+                const int b0 = s - kPer * lane;  // this lane's entries done
+                out &= here & (b0 <= 0 ? 0xFFu : b0 >= kPer ? 0u : 0xFFu << b0);
+                // the first entry that ends the run (cnt: none)
+                const int f = (int)__reduce_min_sync(
+                    kFull, out ? (unsigned)(kPer * lane + __ffs(out) - 1) : (unsigned)cnt);
+                if (f > s) {  // entries s .. f - 1 (A == 2^53 carries into the exponent)
+                    const int64_t w = (H.P[(f - 1) & 7][(f - 1) >> 3] ^ sg) + base + 1;
+                    acc = __longlong_as_double(
+                        (long long)((ab & ~((uint64_t)kChainOne - 1)) + (uint64_t)w));
+                    s = f;
+                }
+                if (s >= cnt) break;
+                run = 1;
+            }
+            // the entry that ended the run; kRunSeq in all where the sum is
+            // left small against its term (exponents compared as integers: the
+            // fp64 pipe is the chain's)
+            ep = T.e[s & 7][s >> 3] - 1023;
+            acc = fma(T.v[s & 7][s >> 3], T.x[s & 7][s >> 3], acc);
+            s++;
+            if (run == 1 && ((__double2hiint(acc) >> 20) & 0x7FF) >= ep + 2) continue;
+            const int e = min(cnt, s + kRunSeq - 1);
+            double pv[kRunSeq - 1], px[kRunSeq - 1];
+#pragma unroll
+            for (int r = 0; r < kRunSeq - 1; r++) {
+                const int i = min(s + r, kTile - 1);
+                pv[r] = T.v[i & 7][i >> 3];
+                px[r] = T.x[i & 7][i >> 3];
+            }
+#pragma unroll
+            for (int r = 0; r < kRunSeq - 1; r++)
+                if (s + r < e) acc = fma(pv[r], px[r], acc);
+            s = e;
+        }
+        if (lane == 0) s_E[t & 1] = (__double2hiint(acc) >> 20) & 0x7FF;
+    }
+    if (threadIdx.x == 0) y[lrow[blockIdx.x]] = acc;
 }
 
 __global__ void k_sp_long_flags(int64_t n, const int32_t *len, int32_t *flag) {
@@ -303,10 +498,27 @@ __global__ void k_sp_long_scatter(int64_t n, const int32_t *flag, const int64_t 
     if (r < n && flag[r]) lrow[idx[r]] = (int32_t)r;
 }
 
-// One warp per long row: its entries copied in CSR order.
-__global__ void k_sp_long_fill(int64_t nlong, const int32_t *lrow, const int64_t *lptr,
+// Block per slice of 32 long rows (longest first), lane per row, the block's
+// warps over the groups of four entries.
+__global__ void k_sp_long_fill(int64_t nrows, const int32_t *lrow, const int64_t *moff,
                                const int32_t *llen, const int64_t *rp, const int32_t *col,
                                const double *val, int32_t *lcol, double *lval) {
+    const int64_t i = (int64_t)blockIdx.x * kSpC + (threadIdx.x & 31);
+    if (i >= nrows) return;
+    const int64_t src = rp[lrow[i]], dst = moff[blockIdx.x] + 4 * (threadIdx.x & 31);
+    const int32_t len = llen[i];
+    for (int32_t g = threadIdx.x >> 5; 4 * g < len; g += blockDim.x >> 5) {
+        for (int k = 0; k < 4 && 4 * g + k < len; k++) {
+            lcol[dst + (int64_t)g * 4 * kSpC + k] = col[src + 4 * g + k];
+            lval[dst + (int64_t)g * 4 * kSpC + k] = val[src + 4 * g + k];
+        }
+    }
+}
+
+// One warp per hub row: its entries copied in CSR order.
+__global__ void k_sp_hub_fill(int64_t nlong, const int32_t *lrow, const int64_t *lptr,
+                              const int32_t *llen, const int64_t *rp, const int32_t *col,
+                              const double *val, int32_t *lcol, double *lval) {
     const int lane = threadIdx.x & 31;
     const int64_t w0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -317,6 +529,18 @@ __global__ void k_sp_long_fill(int64_t nlong, const int32_t *lrow, const int64_t
             lval[dst + k] = val[src + k];
         }
     }
+}
+
+// Rows longer than this have a CTA each. Lane per row does 32 rows at once
+// but takes about 70 ns per entry of its longest; a hub takes 3 ns per entry
+// and, for signed terms, about 0.35 us at each of its some 10 sqrt(N) entries
+// that leave the binade, whatever the other rows are. So the line is drawn
+// where the longest lane-per-row chain ends well before the longest hub's, and
+// not lower: R-MAT scale 22 (longest row 163,186) takes 2.12 ms at 25 sqrt(N)
+// and at 12, 4.16 at 6, where 9,109 rows are hubs and their CTAs run in
+// waves; with positive terms 0.94, 0.84 and 1.25 ms.
+int32_t hub_threshold(int32_t longest) {
+    return std::max<int32_t>(kSpLong, (int32_t)(12.0 * std::sqrt((double)longest)));
 }
 
 alb_status build(alb_sellmat *m, const int64_t *rowptr, const int32_t *col, const double *val) {
@@ -345,6 +569,11 @@ alb_status build(alb_sellmat *m, const int64_t *rowptr, const int32_t *col, cons
         bool sorted = true;
         ALB_TRY(csr_check(n, d_rp, d_col, nnz, st, &sorted));
         m->nslices = (n + kSpC - 1) / kSpC;
+        // up to two slices for each quarter of an SM there is nothing to
+        // balance, and index order is the faster one (n = 20,011: 11.9
+        // against 13.9 us; at 131,072: 14.2 against 12.2)
+        m->wslices = m->nslices > 8 * (int64_t)m->num_sms && m->sigma % kSpC == 0
+                         ? m->sigma / kSpC : 1;
         const int64_t npad = m->nslices * kSpC;
         ALB_TRY(dmalloc((void **)&len, sizeof(int32_t) * (size_t)n, "SpMV lengths"));
         ALB_TRY(dmalloc((void **)&m->perm, sizeof(int32_t) * (size_t)n, "SpMV order"));
@@ -407,12 +636,22 @@ alb_status build(alb_sellmat *m, const int64_t *rowptr, const int32_t *col, cons
             std::vector<int32_t> srow((size_t)nl), slen((size_t)nl);
             std::vector<int64_t> sptr((size_t)nl + 1, 0);
             for (int64_t i = 0; i < nl; i++) {
-                const int64_t len = hlen[(size_t)order[(size_t)i]];
                 srow[(size_t)i] = hrow[(size_t)order[(size_t)i]];
-                slen[(size_t)i] = (int32_t)len;
-                sptr[(size_t)i + 1] = sptr[(size_t)i] + ((len + kLb - 1) / kLb) * kLb;
+                slen[(size_t)i] = (int32_t)hlen[(size_t)order[(size_t)i]];
             }
-            m->max_long = slen[0];
+            m->nhub = std::lower_bound(slen.begin(), slen.end(), hub_threshold(slen[0]),
+                                       std::greater<int32_t>()) -
+                      slen.begin();
+            // hubs: rows one after the other, each padded to kLb entries; the
+            // others: slices of 32 rows, as wide as the first (longest) one
+            for (int64_t i = 0; i < m->nhub; i++)
+                sptr[(size_t)i + 1] = sptr[(size_t)i] + ((slen[(size_t)i] + kLb - 1) / kLb) * kLb;
+            int64_t nent = (sptr[(size_t)m->nhub] + 127) & ~127ll;
+            const int64_t nmid = (nl - m->nhub + kSpC - 1) / kSpC;
+            for (int64_t q = 0; q < nmid; q++) {
+                sptr[(size_t)(m->nhub + q)] = nent;
+                nent += (int64_t)kSpC * (((int64_t)slen[(size_t)(m->nhub + q * kSpC)] + kLb - 1) / kLb) * kLb;
+            }
             ALB_TRY(dmalloc((void **)&m->llen, sizeof(int32_t) * (size_t)nl, "SpMV long lengths"));
             ALB_CK(cudaMemcpyAsync(m->lrow, srow.data(), sizeof(int32_t) * (size_t)nl,
                                    cudaMemcpyHostToDevice, st));
@@ -422,13 +661,17 @@ alb_status build(alb_sellmat *m, const int64_t *rowptr, const int32_t *col, cons
                                    cudaMemcpyHostToDevice, st));
             // padded entries are never summed; zeroed so that the layout is
             // fixed by the CSR alone
-            const int64_t nent = sptr[(size_t)nl];
             ALB_TRY(dmalloc((void **)&m->lcol, sizeof(int32_t) * (size_t)nent, "SpMV long columns"));
             ALB_TRY(dmalloc((void **)&m->lval, sizeof(double) * (size_t)nent, "SpMV long values"));
             ALB_CK(cudaMemsetAsync(m->lcol, 0, sizeof(int32_t) * (size_t)nent, st));
             ALB_CK(cudaMemsetAsync(m->lval, 0, sizeof(double) * (size_t)nent, st));
-            k_sp_long_fill<<<blocks_for(nl * 32, 256), 256, 0, st>>>(
-                nl, m->lrow, m->lptr, m->llen, d_rp, d_col, d_val, m->lcol, m->lval);
+            if (m->nhub > 0)
+                k_sp_hub_fill<<<blocks_for(m->nhub * 32, 256), 256, 0, st>>>(
+                    m->nhub, m->lrow, m->lptr, m->llen, d_rp, d_col, d_val, m->lcol, m->lval);
+            if (nmid > 0)
+                k_sp_long_fill<<<(unsigned)nmid, 256, 0, st>>>(
+                    nl - m->nhub, m->lrow + m->nhub, m->lptr + m->nhub, m->llen + m->nhub, d_rp,
+                    d_col, d_val, m->lcol, m->lval);
             ALB_CK(cudaGetLastError());
             // the host vectors must outlive the copies
             ALB_CK(cudaStreamSynchronize(st));
@@ -459,45 +702,49 @@ void destroy(alb_sellmat *m) {
     dfree(m->lval);
     dfree(m->llen);
     if (m->side) cudaStreamSynchronize(m->side);
+    if (m->side2) cudaStreamSynchronize(m->side2);
     if (m->ev0) cudaEventDestroy(m->ev0);
     if (m->ev1) cudaEventDestroy(m->ev1);
     if (m->fork) cudaEventDestroy(m->fork);
     if (m->join) cudaEventDestroy(m->join);
+    if (m->join2) cudaEventDestroy(m->join2);
     if (m->stream) cudaStreamDestroy(m->stream);
     if (m->side) cudaStreamDestroy(m->side);
+    if (m->side2) cudaStreamDestroy(m->side2);
     cudaGetLastError();
     if (prev >= 0) cudaSetDevice(prev);
     delete m;
 }
 
 alb_status launch(alb_sellmat *m, const double *d_x, double *d_y, float *us) {
-    int per = 0, sms = 0;
-    ALB_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_spmv, kSpBlock, 0));
-    ALB_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device));
-    const int64_t want = (m->nslices + 15) / 16;  // 16 warps a block, one slice each
-    const int64_t cap = (int64_t)(per > 0 ? per : 2) * sms;
+    const int per = resident_blocks((const void *)k_spmv, kSpBlock);
+    const int64_t want = (m->nslices + kSpBlock / 32 - 1) / (kSpBlock / 32);  // one slice a warp
+    const int64_t cap = (int64_t)(per > 0 ? per : 2) * m->num_sms;
     const unsigned grid = (unsigned)std::max<int64_t>(1, std::min(want, cap));
     if (us) ALB_CK(cudaEventRecord(m->ev0, m->stream));
-    // the long rows' chains (one dependent fma per entry, the longest row
-    // the critical path) start first, and the slices run beside them
-    if (m->nlong > 0) {
-        ALB_CK(cudaEventRecord(m->fork, m->stream));
+    // the long rows first: their chains are the longest of the launch
+    const bool hubs = m->nhub > 0, rest = m->nlong > m->nhub;
+    if (hubs || rest) ALB_CK(cudaEventRecord(m->fork, m->stream));
+    if (hubs) {
         ALB_CK(cudaStreamWaitEvent(m->side, m->fork, 0));
-        // the few longest rows on CTAs of their own (side stream); the other
-        // long rows, then the slices, on the main stream beside them
-        const int64_t nsolo = std::min<int64_t>(m->nlong, kSoloRows);
-        k_spmv_long<true><<<(unsigned)nsolo, kSoloThreads, 0, m->side>>>(
-            m->nlong, 0, m->lrow, m->lptr, m->llen, m->lcol, m->lval, d_x, d_y);
+        k_spmv_hub<<<(unsigned)m->nhub, kHubThreads, 0, m->side>>>(
+            m->lrow, m->lptr, m->llen, m->lcol, m->lval, d_x, d_y);
         ALB_CK(cudaGetLastError());
         ALB_CK(cudaEventRecord(m->join, m->side));
-        if (m->nlong > nsolo)
-            k_spmv_long<false><<<blocks_for(m->nlong - nsolo, 32), kSpLongBlock, 0, m->stream>>>(
-                m->nlong, nsolo, m->lrow, m->lptr, m->llen, m->lcol, m->lval, d_x, d_y);
     }
-    k_spmv<<<grid, kSpBlock, 0, m->stream>>>(m->n, m->nslices, m->perm, m->deg, m->slice_off, m->col,
-                                         m->val, d_x, d_y);
+    if (rest) {
+        ALB_CK(cudaStreamWaitEvent(m->side2, m->fork, 0));
+        k_spmv_long<<<blocks_for(m->nlong - m->nhub, kSpC), kSpLongBlock, 0, m->side2>>>(
+            m->nlong - m->nhub, m->lrow + m->nhub, m->lptr + m->nhub, m->llen + m->nhub, m->lcol,
+            m->lval, d_x, d_y);
+        ALB_CK(cudaGetLastError());
+        ALB_CK(cudaEventRecord(m->join2, m->side2));
+    }
+    k_spmv<<<grid, kSpBlock, 0, m->stream>>>(m->n, m->nslices, m->wslices, m->perm, m->deg,
+                                             m->slice_off, m->col, m->val, d_x, d_y);
     ALB_CK(cudaGetLastError());
-    if (m->nlong > 0) ALB_CK(cudaStreamWaitEvent(m->stream, m->join, 0));
+    if (hubs) ALB_CK(cudaStreamWaitEvent(m->stream, m->join, 0));
+    if (rest) ALB_CK(cudaStreamWaitEvent(m->stream, m->join2, 0));
     if (us) {
         ALB_CK(cudaEventRecord(m->ev1, m->stream));
         ALB_CK(cudaEventSynchronize(m->ev1));
@@ -529,12 +776,16 @@ alb_status alb_sellmat_create(int64_t n, const int64_t *rowptr, const int32_t *c
     m->nnz = rowptr[n];
     m->sigma = sigma;
     cudaError_t e = cudaGetDevice(&m->device);
+    if (e == cudaSuccess)
+        e = cudaDeviceGetAttribute(&m->num_sms, cudaDevAttrMultiProcessorCount, m->device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreate(&m->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&m->ev1);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&m->side, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&m->fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&m->join, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&m->side2, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&m->join2, cudaEventDisableTiming);
     if (e != cudaSuccess) {
         cudaGetLastError();
         destroy(m);
