@@ -27,6 +27,7 @@
 #include <new>
 #include <vector>
 
+#include "bfs_cluster.h"
 #include "graph.h"
 #include "selector.cuh"
 
@@ -989,12 +990,6 @@ __global__ void k_init_bulk(BfsArgs a) {
     }
 }
 
-struct InitParams {
-    int32_t root, policy, trace_cap, level_cap;
-    float alpha, beta, mean_deg, skew;
-    int64_t n_live, m_in, active0;
-};
-
 __global__ void k_init_root(BfsArgs a, InitParams ip) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     const int32_t rp = a.inv[ip.root];
@@ -1783,6 +1778,41 @@ alb_status run_persistent(alb_graph *g, const BfsArgs &a) {
 }
 
 
+// Waits for the traversal and fills in its statistics from the control
+// block's host copy. kernels: launches made by the host; loop_counts: plus
+// those the level loop counted.
+alb_status finish_call(alb_graph *g, const alb_bfs_opts &o, const std::vector<float> &step_us,
+                       int64_t kernels, bool loop_counts, alb_stats *st) {
+    ALB_CK(cudaStreamSynchronize(g->stream));
+    const BfsCtl &c = *g->bfs.h_ctl;
+    if (c.err) return fail(c.err, "BFS aborted on the device (code %d)", c.err);
+    if (!c.done) return fail(ALB_ERR_DEVICE, "BFS level loop ended without finishing");
+    float ms = 0;
+    ALB_CK(cudaEventElapsedTime(&ms, g->ev0, g->ev1));
+    g->last_trace_valid = false;
+    if (o.trace) {
+        const int32_t cnt = std::min(c.trace_len, g->bfs.trace_cap);
+        g->last_trace.resize((size_t)cnt);
+        if (cnt)
+            ALB_CK(cudaMemcpy(g->last_trace.data(), g->bfs.trace, sizeof(alb_level_rec) * cnt,
+                              cudaMemcpyDeviceToHost));
+        for (int32_t i = 0; i < cnt && i < (int32_t)step_us.size(); i++)
+            g->last_trace[i].step_us = step_us[i];
+        g->last_trace_valid = true;
+    }
+    if (st) {
+        st->num_levels = c.level;
+        st->levels_topdown = c.levels_td;
+        st->levels_bottomup = c.levels_bu;
+        st->pushed_roots = 0;
+        st->reached = c.reached;
+        st->edges = c.edges;
+        st->ms = ms;
+        st->kernels = kernels + (loop_counts ? c.launches : 0);
+    }
+    return ALB_OK;
+}
+
 alb_status bfs_impl(alb_graph *g, int32_t root, const alb_bfs_opts &o, int32_t *d_level,
                     int32_t *d_parent, alb_stats *st) {
     ALB_TRY(bfs_scratch_alloc(g));
@@ -1802,7 +1832,14 @@ alb_status bfs_impl(alb_graph *g, int32_t root, const alb_bfs_opts &o, int32_t *
     ip.m_in = s.m_in;
     ip.active0 = s.active0;
     const Launch wide = level_launch(g, 256);
+    const bool small = cluster_takes(g, o, a);
     ALB_CK(cudaEventRecord(g->ev0, stream));
+    if (small) {
+        g->bfs.h_ctl->done = g->bfs.h_ctl->err = 0;
+        ALB_TRY(cluster_launch(a, ip, d_level, d_parent, g->bfs.h_ctl, stream));
+        ALB_CK(cudaEventRecord(g->ev1, stream));
+        return finish_call(g, o, {}, 1, false, st);
+    }
     k_init_bulk<<<wide.grid, wide.block, 0, stream>>>(a);
     k_init_root<<<1, 32, 0, stream>>>(a, ip);
     ALB_CK(cudaGetLastError());
@@ -1838,39 +1875,11 @@ alb_status bfs_impl(alb_graph *g, int32_t root, const alb_bfs_opts &o, int32_t *
     ALB_CK(cudaGetLastError());
     ALB_CK(cudaEventRecord(g->ev1, stream));
     ALB_CK(cudaMemcpyAsync(g->bfs.h_ctl, a.ctl, sizeof(BfsCtl), cudaMemcpyDeviceToHost, stream));
-    ALB_CK(cudaStreamSynchronize(stream));
-    const BfsCtl &c = *g->bfs.h_ctl;
-    if (c.err) return fail(c.err, "BFS aborted on the device (code %d)", c.err);
-    if (!c.done) return fail(ALB_ERR_DEVICE, "BFS level loop ended without finishing");
-    float ms = 0;
-    ALB_CK(cudaEventElapsedTime(&ms, g->ev0, g->ev1));
-    g->last_trace_valid = false;
-    if (o.trace) {
-        const int32_t cnt = std::min(c.trace_len, g->bfs.trace_cap);
-        g->last_trace.resize((size_t)cnt);
-        if (cnt)
-            ALB_CK(cudaMemcpy(g->last_trace.data(), g->bfs.trace, sizeof(alb_level_rec) * cnt,
-                              cudaMemcpyDeviceToHost));
-        for (int32_t i = 0; i < cnt && i < (int32_t)step_us.size(); i++)
-            g->last_trace[i].step_us = step_us[i];
-        g->last_trace_valid = true;
-    }
-    if (st) {
-        st->num_levels = c.level;
-        st->levels_topdown = c.levels_td;
-        st->levels_bottomup = c.levels_bu;
-        st->pushed_roots = 0;
-        st->reached = c.reached;
-        st->edges = c.edges;
-        st->ms = ms;
-        // init_bulk + init_root (+ scatter), plus the loop's own launches
-        st->kernels = 2 + ((d_level || d_parent) ? 1 : 0) +
-                      (o.loop == ALB_LOOP_PERSISTENT ? 1 : c.launches);
-    }
-    return ALB_OK;
+    // init_bulk + init_root (+ scatter), plus the loop's own launches
+    const bool counted = o.loop != ALB_LOOP_PERSISTENT;
+    const int64_t kernels = 2 + ((d_level || d_parent) ? 1 : 0) + (counted ? 0 : 1);
+    return finish_call(g, o, step_us, kernels, counted, st);
 }
-
-// Launch the step kernels of one variant for the current level.
 
 // Device copies of the state a level step mutates (restored between variants).
 struct LevelSnapshot {

@@ -266,15 +266,34 @@ struct BfsArgs {
     int32_t withhold_level, withhold_block, short_bulk;
 };
 
+// Initial values of a traversal.
+struct InitParams {
+    int32_t root, policy, trace_cap, level_cap;
+    float alpha, beta, mean_deg, skew;
+    int64_t n_live, m_in, active0;
+};
+
 // Shared by host and device: pick the direction for the current level.
+// mf > mu / alpha, nf > n / beta and the reference's threshold are decided in
+// fp64; on the device a single fp64 operation takes some 115 cycles and a
+// division twenty times that, so fp32 decides first where the two sides are
+// further apart than its rounding (three operations, each within 2^-23).
+__host__ __device__ inline bool above_quotient(int64_t x, int64_t y, float q) {
+#ifdef __CUDA_ARCH__
+    const float l = (float)x, r = __fdividef((float)y, q);
+    if (l > r * 1.0001f) return true;
+    if (l < r * 0.9999f) return false;
+#endif
+    return (double)x > (double)y / (double)q;
+}
+
 __host__ __device__ inline int beamer_dir(const BfsCtl &c) {
     if (c.prev_dir < 0 || c.prev_dir == ALB_DIR_TOPDOWN) {
         // top-down -> bottom-up when the frontier's edges exceed m_u / alpha
-        return ((double)c.mf > (double)c.mu / (double)c.alpha) ? ALB_DIR_BOTTOMUP
-                                                               : ALB_DIR_TOPDOWN;
+        return above_quotient(c.mf, c.mu, c.alpha) ? ALB_DIR_BOTTOMUP : ALB_DIR_TOPDOWN;
     }
     // stay bottom-up while the frontier grows or is large
-    bool stay = (c.nf >= c.prev_nf) || ((double)c.nf > (double)c.n / (double)c.beta);
+    bool stay = (c.nf >= c.prev_nf) || above_quotient(c.nf, c.n, c.beta);
     return stay ? ALB_DIR_BOTTOMUP : ALB_DIR_TOPDOWN;
 }
 

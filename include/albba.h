@@ -149,7 +149,9 @@ alb_status alb_sell_long_export(const alb_graph *g, int64_t *nlong, int32_t *lro
                                   (level 0 runs top-down) */
 #define ALB_POLICY_BOTTOMUP_NOBYPASS 5 /* bottom-up pull, no slice bypass */
 
-/* Level-loop driver. */
+/* Level-loop driver. Small graphs (up to 2^18 vertices with the graph loop,
+ * 2^17 with the persistent one) run as one launch of one thread-block cluster
+ * under either device-driven loop, unless a trace is asked for. */
 #define ALB_LOOP_HOST 0       /* one set of launches per level, host decides */
 #define ALB_LOOP_GRAPH 1      /* CUDA graph with a device-driven while node */
 #define ALB_LOOP_PERSISTENT 2 /* one cooperative kernel for all levels */
