@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "bfs_cluster.h"
+#include "bfs_grid.h"
 #include "graph.h"
 #include "selector.cuh"
 
@@ -1451,6 +1452,8 @@ alb_status bfs_scratch_alloc(alb_graph *g) {
     ALB_TRY(dmalloc((void **)&b.parent_pos, sizeof(uint32_t) * n, "parents"));
     ALB_TRY(dmalloc((void **)&b.ctl, sizeof(BfsCtl), "level control"));
     ALB_TRY(dmalloc((void **)&b.bar, 256, "grid barrier"));
+    ALB_CK(cudaMemsetAsync(b.bar, 0, 256, g->stream));
+    ALB_TRY(dmalloc(&b.slots, sizeof(GridSlots), "level counters"));
     b.trace_cap = (int32_t)std::min<int64_t>(n + 2, 1 << 16);
     ALB_TRY(dmalloc((void **)&b.trace, sizeof(alb_level_rec) * b.trace_cap, "level trace"));
     ALB_CK(cudaMallocHost((void **)&b.h_ctl, sizeof(BfsCtl)));
@@ -1471,6 +1474,8 @@ void bfs_scratch_free(alb_graph *g) {
     dfree(b.out_parent);
     dfree(b.ctl);
     dfree(b.bar);
+    dfree(b.slots);
+    dfree(b.vrec);
     dfree(b.trace);
     if (b.h_ctl) cudaFreeHost(b.h_ctl);
     b = BfsScratch();
@@ -1784,7 +1789,10 @@ alb_status run_persistent(alb_graph *g, const BfsArgs &a) {
 alb_status finish_call(alb_graph *g, const alb_bfs_opts &o, const std::vector<float> &step_us,
                        int64_t kernels, bool loop_counts, alb_stats *st) {
     ALB_CK(cudaStreamSynchronize(g->stream));
-    const BfsCtl &c = *g->bfs.h_ctl;
+    BfsCtl &c = *g->bfs.h_ctl;
+    // a block that left early wrote its results before the others gave up
+    if (!c.done && !c.err)
+        ALB_CK(cudaMemcpy(&c.err, &g->bfs.ctl->err, sizeof(c.err), cudaMemcpyDeviceToHost));
     if (c.err) return fail(c.err, "BFS aborted on the device (code %d)", c.err);
     if (!c.done) return fail(ALB_ERR_DEVICE, "BFS level loop ended without finishing");
     float ms = 0;
@@ -1840,13 +1848,16 @@ alb_status bfs_impl(alb_graph *g, int32_t root, const alb_bfs_opts &o, int32_t *
         ALB_CK(cudaEventRecord(g->ev1, stream));
         return finish_call(g, o, {}, 1, false, st);
     }
-    k_init_bulk<<<wide.grid, wide.block, 0, stream>>>(a);
-    k_init_root<<<1, 32, 0, stream>>>(a, ip);
-    ALB_CK(cudaGetLastError());
+    const bool coop = grid_takes(g, o, a);
+    if (!coop) {
+        k_init_bulk<<<wide.grid, wide.block, 0, stream>>>(a);
+        k_init_root<<<1, 32, 0, stream>>>(a, ip);
+        ALB_CK(cudaGetLastError());
+    }
     // the bitmaps' L2 window applies to the level loop's launches on the
     // stream (the CUDA-graph loop carries it on its kernel nodes); it is
     // removed again before the stream is handed back
-    const bool win = g->bfs.win.num_bytes > 0 && o.loop != ALB_LOOP_GRAPH;
+    const bool win = g->bfs.win.num_bytes > 0 && (coop || o.loop != ALB_LOOP_GRAPH);
     if (win) {
         cudaStreamAttrValue v = {};
         v.accessPolicyWindow = g->bfs.win;
@@ -1854,7 +1865,20 @@ alb_status bfs_impl(alb_graph *g, int32_t root, const alb_bfs_opts &o, int32_t *
     }
     std::vector<float> step_us;
     alb_status lrc = ALB_OK;
-    if (o.loop == ALB_LOOP_HOST) {
+    if (coop) {
+        g->bfs.h_ctl->done = g->bfs.h_ctl->err = 0;
+        if (!g->bfs.vrec_ready) {  // once, on the first call; without memory for them, without
+            g->bfs.vrec_ready = true;
+            if (s.max_deg <= kRecMaxDeg &&
+                dmalloc((void **)&g->bfs.vrec, sizeof(int4) * (size_t)g->n, "push-row records") ==
+                    ALB_OK)
+                lrc = row_recs_launch(g, a, g->bfs.vrec, stream);
+        }
+        const GridArgs x{(GridSlots *)g->bfs.slots, g->bfs.vrec, s.max_deg, s.m_in,
+                         s.m_out, g->symmetric ? 1 : 0,
+                         g->bfs.h_ctl, 0};
+        if (lrc == ALB_OK) lrc = grid_launch(g, a, ip, x, stream);
+    } else if (o.loop == ALB_LOOP_HOST) {
         lrc = run_host_loop(g, a, o, step_us);
     } else if (o.loop == ALB_LOOP_PERSISTENT) {
         lrc = run_persistent(g, a);
@@ -1871,13 +1895,21 @@ alb_status bfs_impl(alb_graph *g, int32_t root, const alb_bfs_opts &o, int32_t *
         cudaStreamSetAttribute(stream, cudaStreamAttributeAccessPolicyWindow, &v);
     }
     ALB_TRY(lrc);
-    if (d_level || d_parent) k_scatter<<<wide.grid, wide.block, 0, stream>>>(a, d_level, d_parent);
+    const bool outputs = d_level || d_parent;
+    if (outputs && scatter_launch(g, a, d_level, d_parent, stream) != ALB_OK)
+        k_scatter<<<wide.grid, wide.block, 0, stream>>>(a, d_level, d_parent);
     ALB_CK(cudaGetLastError());
     ALB_CK(cudaEventRecord(g->ev1, stream));
+    if (coop) {
+        const alb_status rc = finish_call(g, o, step_us, outputs ? 2 : 1, false, st);
+        // (after an error the arrival counter is left between two barriers)
+        if (rc != ALB_OK) ALB_CK(cudaMemsetAsync(g->bfs.bar, 0, 256, stream));
+        return rc;
+    }
     ALB_CK(cudaMemcpyAsync(g->bfs.h_ctl, a.ctl, sizeof(BfsCtl), cudaMemcpyDeviceToHost, stream));
     // init_bulk + init_root (+ scatter), plus the loop's own launches
     const bool counted = o.loop != ALB_LOOP_PERSISTENT;
-    const int64_t kernels = 2 + ((d_level || d_parent) ? 1 : 0) + (counted ? 0 : 1);
+    const int64_t kernels = 2 + (outputs ? 1 : 0) + (counted ? 0 : 1);
     return finish_call(g, o, step_us, kernels, counted, st);
 }
 

@@ -18,8 +18,7 @@
 // level (32-bit counters and few unrolled loops for that reason). Measured
 // against the loops of bfs.cu (CUDA graph / persistent kernel, us a call,
 // Beamer): R-MAT edge factor 16, n = 1,024: 24 (157 / 98), 65,536: 54 (198 /
-// 129), 262,144: 111 (226 / 149); uniform random, mean degree 8, n = 65,536:
-// 83 (326 / 203); grid of 131,044 (307 levels): 1,326 (8,459 / 3,278).
+// 129); uniform random, mean degree 8, n = 65,536: 83 (326 / 203).
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -80,7 +79,7 @@ struct Shared {
     unsigned hit;                 // a cooperative scan's first hit
     int32_t list[kPushRows], list_st[kPushRows], list_off[kPushRows + 1];
     int32_t warp_rows[kWarps], warp_edges[kWarps];
-    __align__(16) float mlp[kMlpParams + 1];
+    MlpCopy mlp;
     List q[2];
 };
 
@@ -583,10 +582,10 @@ __device__ void next_level(Shared &s, const State &t, const BfsArgs &a, const In
     c.feat_mean_deg = in.mean_deg;
     c.feat_skew = in.skew;
     int dir;
-    if (learned && s.mlp[kMlpParams] != 0.0f) {
+    if (learned && s.mlp.loaded()) {
         float f[kMlpIn];
-        level_features(c, f);
-        dir = mlp_select_warp(s.mlp, f);
+        level_features_warp(c, f);
+        dir = s.mlp.select(f);
     } else {
         dir = rule_dir(c);
     }
@@ -626,8 +625,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         a.parent_pos[p] = kFull;
     }
     const bool learned = in.policy == ALB_POLICY_LEARNED && a.mlp;
-    if (learned)
-        for (int i = threadIdx.x; i <= kMlpParams; i += kThreads) s.mlp[i] = a.mlp[i];
+    if (learned) s.mlp.load(a.mlp);
     if (threadIdx.x < 8) reinterpret_cast<unsigned *>(s.cnt)[threadIdx.x] = 0;
     __syncthreads();
     State t;
@@ -799,8 +797,7 @@ bool cluster_ready(int device) {
 
 bool cluster_takes(const alb_graph *g, const alb_bfs_opts &o, const BfsArgs &a) {
     // (counters are 32 bits wide)
-    const int64_t limit = o.loop == ALB_LOOP_GRAPH ? kClusterMaxN : kClusterMaxPersistent;
-    return g->n <= limit && g->sell.m_in <= INT32_MAX && g->sell.m_out <= INT32_MAX && o.loop != ALB_LOOP_HOST && !o.trace &&
+    return g->n <= kClusterMaxN && g->sell.m_in <= INT32_MAX && g->sell.m_out <= INT32_MAX && o.loop != ALB_LOOP_HOST && !o.trace &&
            o.policy != ALB_POLICY_BOTTOMUP_NOBYPASS && a.withhold_level < 0 && !a.short_bulk &&
            cluster_ready(g->device);
 }

@@ -6,14 +6,13 @@
 
 namespace alb {
 
-// Largest graph (vertices) the cluster kernel takes: three bitmaps of it fit
-// in one CTA's shared memory beside the kernel's 75 KB. In place of the
-// persistent kernel it is taken up to half of that: at 262,144 vertices, 16 SMs
-// lose to 152 where the learned policy pushes dense frontiers (R-MAT 194
-// against 148 us, uniform random 272 against 216), at 131,072 they win (125
-// against 137, 189 against 211). The CUDA-graph loop loses at either size.
-constexpr int64_t kClusterMaxN = 1 << 18;
-constexpr int64_t kClusterMaxPersistent = 1 << 17;
+// Largest graph (vertices) the cluster kernel takes. Against the cooperative
+// kernel on all SMs (bfs_grid.cu), us a call, Beamer / learned: R-MAT edge
+// factor 16, n = 65,536: 65 / 87 against 77 / 91, at 131,072: 87 / 135 against
+// 82 / 100; grid of 65,536: 968 / 1,447 against 1,186 / 1,793, of 131,044:
+// 1,392 / 1,617 against 1,256 / 1,240; uniform random, mean degree 8, 32,768:
+// 62 / 109 against 82 / 84, 65,536: 93 / 149 against 85 / 94.
+constexpr int64_t kClusterMaxN = 1 << 16;
 
 // Whether the call runs as one cluster launch. Calls that ask for what only
 // the other loops have keep them: per-level traces, host-driven levels, the

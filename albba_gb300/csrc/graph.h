@@ -97,6 +97,9 @@ struct BfsScratch {
     BfsCtl *ctl = nullptr;
     BfsCtl *h_ctl = nullptr;  // pinned mirror
     unsigned long long *bar = nullptr;  // persistent-kernel grid barrier
+    void *slots = nullptr;              // counters of the cooperative kernel (GridSlots)
+    int4 *vrec = nullptr;               // its push-row records (null: none)
+    bool vrec_ready = false;
     alb_level_rec *trace = nullptr;
     int32_t trace_cap = 0;
 };

@@ -63,12 +63,14 @@ __host__ __device__ inline int argmin3(const float *o) {
 // the argmin variant. Must be called by a full warp. Each lane first issues
 // all of its parameter loads (its rows of W1 and W2 as 16-byte loads, its
 // biases, its column of W3), so the pass costs one memory round trip rather
-// than one per layer; P must be 16-byte aligned (the parameter blocks are).
-// P may point to global memory or to a shared-memory copy (generic loads).
-__device__ inline int mlp_select_warp(const float *P, const float *x) {
+// than one per layer. W1 and W2 lie kS1 and kS2 floats a row; P holds the rest
+// at its usual place. All 16-byte aligned (the parameter blocks are).
+template <int kS1 = kMlpIn, int kS2 = kMlpH>
+__device__ inline int mlp_select_rows(const float *W1, const float *W2, const float *P,
+                                      const float *x) {
     const int j = threadIdx.x & 31;
-    const float4 *w1 = reinterpret_cast<const float4 *>(P + kMlpW1 + j * kMlpIn);
-    const float4 *w2 = reinterpret_cast<const float4 *>(P + kMlpW2 + j * kMlpH);
+    const float4 *w1 = reinterpret_cast<const float4 *>(W1 + j * kS1);
+    const float4 *w2 = reinterpret_cast<const float4 *>(W2 + j * kS2);
     float4 r1[kMlpIn / 4], r2[kMlpH / 4];
 #pragma unroll
     for (int i = 0; i < kMlpIn / 4; i++) r1[i] = w1[i];
@@ -98,6 +100,47 @@ __device__ inline int mlp_select_warp(const float *P, const float *x) {
 #pragma unroll
     for (int k = 0; k < kMlpOut; k++) o[k] = warp_sum(w3[k] * h2) + b3[k];
     return argmin3(o);
+}
+
+// P may point to global memory or to a shared-memory copy (generic loads).
+__device__ inline int mlp_select_warp(const float *P, const float *x) {
+    return mlp_select_rows(P + kMlpW1, P + kMlpW2, P, x);
+}
+
+// A copy of the parameters in shared memory whose rows start in different
+// banks (as stored, the 32 lanes' rows of W2 all start in one).
+struct MlpCopy {
+    static constexpr int kS1 = kMlpIn + 4, kS2 = kMlpH + 4;
+    __align__(16) float w1[kMlpH * kS1];
+    float w2[kMlpH * kS2];
+    float rest[kMlpParams + 1];  // biases and W3, and whether weights are loaded
+    // all threads of a block
+    __device__ __forceinline__ void load(const float *P) {
+        for (int i = threadIdx.x; i <= kMlpParams; i += blockDim.x) {
+            const float v = P[i];
+            rest[i] = v;
+            if (i < kMlpB1) w1[i / kMlpIn * kS1 + i % kMlpIn] = v;
+            if (i >= kMlpW2 && i < kMlpB2)
+                w2[(i - kMlpW2) / kMlpH * kS2 + (i - kMlpW2) % kMlpH] = v;
+        }
+    }
+    __device__ __forceinline__ bool loaded() const { return rest[kMlpParams] != 0.0f; }
+    __device__ __forceinline__ int select(const float *x) const {
+        return mlp_select_rows<kS1, kS2>(w1, w2, rest, x);
+    }
+};
+
+// level_features, one feature a lane.
+__device__ inline void level_features_warp(const BfsCtl &c, float *f) {
+    const int i = threadIdx.x & 31;
+    const int64_t n = i == 0 ? c.nf : i == 1 ? c.mf : i == 2 ? c.nu : c.mu;
+    float v = log2f(1.0f + (i == 5 ? c.feat_mean_deg : (float)n)) *
+              (i == 5 ? 1.0f / 8.0f : 1.0f / 32.0f);
+    if (i == 4) v = fminf((float)c.level, 256.0f) * (1.0f / 64.0f);
+    if (i == 6) v = c.feat_skew * (1.0f / 16.0f);
+    if (i == 7) v = c.nwords > 0 ? (float)c.active_words / (float)c.nwords : 0.0f;
+#pragma unroll
+    for (int k = 0; k < kMlpIn; k++) f[k] = __shfl_sync(kFull, v, k);
 }
 #endif
 

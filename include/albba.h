@@ -149,9 +149,11 @@ alb_status alb_sell_long_export(const alb_graph *g, int64_t *nlong, int32_t *lro
                                   (level 0 runs top-down) */
 #define ALB_POLICY_BOTTOMUP_NOBYPASS 5 /* bottom-up pull, no slice bypass */
 
-/* Level-loop driver. Small graphs (up to 2^18 vertices with the graph loop,
- * 2^17 with the persistent one) run as one launch of one thread-block cluster
- * under either device-driven loop, unless a trace is asked for. */
+/* Level-loop driver. Single-root searches under either device-driven loop run
+ * as one kernel for all levels (graphs of up to 2^16 vertices on one
+ * thread-block cluster, larger ones on all SMs), except where a trace or the
+ * pull without bypass is asked for: those, and the batched searches, run as
+ * described here. */
 #define ALB_LOOP_HOST 0       /* one set of launches per level, host decides */
 #define ALB_LOOP_GRAPH 1      /* CUDA graph with a device-driven while node */
 #define ALB_LOOP_PERSISTENT 2 /* one cooperative kernel for all levels */

@@ -38,7 +38,7 @@ def _random(n, m, seed, hubs=0):
 
 
 @pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 1023, 1024, 1025, 2049, 4097, 8191, 16385, 40001,
-                               (1 << 18) - 1, 1 << 18, (1 << 18) + 1])
+                               (1 << 16) - 1, 1 << 16, (1 << 16) + 1])
 def test_sizes_every_policy(n):
     g = _random(n, 4 * n, n, hubs=2 if n > 4000 else 0)
     roots = [0, n // 2, n - 1]
