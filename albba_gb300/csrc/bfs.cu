@@ -1874,8 +1874,8 @@ alb_status bfs_impl(alb_graph *g, int32_t root, const alb_bfs_opts &o, int32_t *
                     ALB_OK)
                 lrc = row_recs_launch(g, a, g->bfs.vrec, stream);
         }
-        const GridArgs x{(GridSlots *)g->bfs.slots, g->bfs.vrec, s.max_deg, s.m_in,
-                         s.m_out, g->symmetric ? 1 : 0,
+        const GridArgs x{(GridSlots *)g->bfs.slots, g->bfs.vrec, s.max_deg, s.m_out,
+                         g->symmetric ? 1 : 0,
                          g->bfs.h_ctl, 0};
         if (lrc == ALB_OK) lrc = grid_launch(g, a, ip, x, stream);
     } else if (o.loop == ALB_LOOP_HOST) {

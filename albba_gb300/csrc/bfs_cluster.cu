@@ -27,6 +27,7 @@
 #include <mutex>
 
 #include "bfs_cluster.h"
+#include "block_push.cuh"
 #include "graph.h"
 #include "selector.cuh"
 
@@ -38,8 +39,6 @@ namespace cg = cooperative_groups;
 constexpr int kThreads = 1024, kWarps = kThreads / 32;
 constexpr int kMaxCtas = 16;
 constexpr int kPullWords = 2;    // words a warp pulls at a time
-// Rows a CTA pushes together: all set bits of kPushWords bitmap words.
-constexpr int kPushWords = 64, kPushRows = kPushWords * 32, kRowsPer = kPushRows / kThreads;
 // Frontiers of at most this many rows are walked by every CTA, each taking
 // its share of the rows longer than kBigRow; in larger ones a row's edges
 // stay with the CTA that owns it.
@@ -72,13 +71,11 @@ struct Shared {
     unsigned nf, mf;
     Counts cnt[2];                // by level parity: what this CTA found
     unsigned next_word;
-    int nlist;                    // rows in list: frontier rows, or long rows left after their head
     unsigned nq[2];               // list counters (rows, edges) by level parity
     int even;                     // the lists are evened out before the level
     unsigned before[kMaxCtas + 1];  // rows in the lists of the CTAs before each
     unsigned hit;                 // a cooperative scan's first hit
-    int32_t list[kPushRows], list_st[kPushRows], list_off[kPushRows + 1];
-    int32_t warp_rows[kWarps], warp_edges[kWarps];
+    PushLists rows;               // frontier rows; or the long rows left after their head
     MlpCopy mlp;
     List q[2];
 };
@@ -122,104 +119,32 @@ __device__ __forceinline__ void push4(const BfsArgs &a, const uint32_t *V, uint3
     }
 }
 
-// This CTA's pushes of the frontier F into its copy N: the rows of kPushWords
-// words at a time (of all words when few rows are split over the CTAs) are
-// listed with the number of edges before each, and the list's edges are dealt
-// out evenly to the CTA's threads, whatever the rows' lengths.
+// This CTA's pushes of the frontier F into its copy N (all words' rows at once
+// when few rows are split over the CTAs).
 __device__ void push_level(const BfsArgs &a, Shared &s, const uint32_t *F, const uint32_t *V,
                            uint32_t *N, int w0, int w1, int rank, int nctas, bool split) {
-    const int lane = lane_id(), wib = threadIdx.x >> 5;
     const int from = split ? 0 : w0, to = split ? (int)a.nwords : w1;
-    const int span = split ? to : kPushWords;
-    for (int b = from; b < to; b += span) {
-        if (threadIdx.x == 0) s.nlist = 0;
-        __syncthreads();
-        for (int w = b + (int)threadIdx.x; w < min(to, b + span); w += kThreads) {
-            uint32_t m = F[w];
-            int at = m ? atomicAdd(&s.nlist, __popc(m)) : 0;
-            for (; m; m &= m - 1) s.list[at++] = w * 32 + __ffs(m) - 1;
-        }
-        __syncthreads();
-        const int rows = s.nlist;
-        if (rows == 0) continue;
-        // rows kRowsPer i .. of thread i; those without edges are dropped
-        int32_t st[kRowsPer], d[kRowsPer], ou[kRowsPer], nd = 0, nr = 0;
-#pragma unroll
-        for (int k = 0; k < kRowsPer; k++) {
-            const int i = kRowsPer * (int)threadIdx.x + k;
-            d[k] = 0;
-            if (i >= rows) continue;
-            int32_t u = s.list[i];
+    block_push<kThreads>(
+        s.rows, F, from, to, split ? to : kPushWords, a.pcol,
+        [&](int32_t u, int32_t &st, int32_t &d, int32_t &ou) {
             ALB_CHECK_ID(u, a.n, 0, &a.ctl->err);
-            st[k] = (int32_t)__ldg(a.prow + u);
-            d[k] = (int32_t)__ldg(a.prow + u + 1) - st[k];
-            ou[k] = __ldg(a.perm + u);
-            if (split) {
-                if (d[k] > kBigRow) {  // this CTA's share
-                    const int32_t per = (d[k] + nctas - 1) / nctas, skip = min(d[k], per * rank);
-                    st[k] += skip;
-                    d[k] = min(per, d[k] - skip);
-                } else if ((u >> 5) < w0 || (u >> 5) >= w1) {
-                    d[k] = 0;
-                }
+            st = (int32_t)__ldg(a.prow + u);
+            d = (int32_t)__ldg(a.prow + u + 1) - st;
+            ou = __ldg(a.perm + u);
+            if (!split) return;
+            if (d > kBigRow) {  // this CTA's share
+                const int32_t per = (d + nctas - 1) / nctas, skip = min(d, per * rank);
+                st += skip;
+                d = min(per, d - skip);
+            } else if ((u >> 5) < w0 || (u >> 5) >= w1) {
+                d = 0;
             }
-            nd += d[k];
-            nr += d[k] > 0;
-        }
-        int32_t at = warp_inclusive_scan(nr), off = warp_inclusive_scan(nd);
-        if (lane == 31) {
-            s.warp_rows[wib] = at;
-            s.warp_edges[wib] = off;
-        }
-        __syncthreads();
-        const int32_t r_inc = warp_inclusive_scan(s.warp_rows[lane]),
-                      e_inc = warp_inclusive_scan(s.warp_edges[lane]);
-        const int32_t R = __shfl_sync(kFull, r_inc, 31), E = __shfl_sync(kFull, e_inc, 31);
-        const int32_t r_b = __shfl_sync(kFull, r_inc, (wib + 31) & 31),
-                      e_b = __shfl_sync(kFull, e_inc, (wib + 31) & 31);
-        at += (wib ? r_b : 0) - nr;
-        off += (wib ? e_b : 0) - nd;
-#pragma unroll
-        for (int k = 0; k < kRowsPer; k++) {
-            if (!d[k]) continue;
-            s.list[at] = ou[k];
-            s.list_st[at] = st[k] - off;  // edge e of the list is pcol[st + e]
-            s.list_off[at] = off;
-            off += d[k];
-            at++;
-        }
-        __syncthreads();
-        // each warp takes a run of edges, 32 at a time (four times over before
-        // the pushes): the rows that start among them make a bit mask, and a
-        // lane's row is the mask's bits up to it further on
-        const int32_t run = ((E + kWarps - 1) / kWarps + 31) & ~31;
-        const int32_t e_end = min(E, run * (wib + 1));
-        int j = 0;
-        if (run * wib < E)
-            for (int step = kPushRows / 2; step > 0; step >>= 1)
-                if (j + step < R && s.list_off[j + step] <= run * wib) j += step;
-        for (int32_t eb = run * wib; eb < e_end; eb += 128) {
-            int32_t v[4];
-            uint32_t ou4[4];
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const int32_t e0 = eb + 32 * k, e = e0 + lane;
-                const int32_t q = j + 1 + lane, rel = q < R ? s.list_off[q] - e0 : 32;
-                const unsigned starts = __reduce_or_sync(kFull, rel < 32 ? 1u << rel : 0u);
-                const int row = j + __popc(starts & (lanemask_lt() | (1u << lane)));
-                v[k] = -1;
-                ou4[k] = 0;
-                if (e < e_end) {
-                    v[k] = __ldg(a.pcol + s.list_st[row] + e);
-                    ALB_CHECK_ID(v[k], a.n, -1, &a.ctl->err);
-                    ou4[k] = (uint32_t)s.list[row];
-                }
-                j += __popc(starts);
-            }
-            push4(a, V, N, v, ou4);
-        }
-        __syncthreads();
-    }
+        },
+        [&](int32_t (&v)[4], const uint32_t (&ou)[4]) {
+            for (int k = 0; k < 4; k++)
+                if (v[k] >= 0) ALB_CHECK_ID(v[k], a.n, -1, &a.ctl->err);
+            push4(a, V, N, v, ou);
+        });
 }
 
 // After the pushes: the CTAs' copies of this CTA's next-frontier words are
@@ -297,7 +222,7 @@ __device__ void pull_long(const BfsArgs &a, Shared &s, const uint32_t *F, const 
         }
         (side ? hi : lo) = b;
     }
-    if (threadIdx.x == 0) s.nlist = 0;
+    if (threadIdx.x == 0) s.rows.nlist = 0;
     __syncthreads();
     for (int i = lo + wib; i < hi; i += kWarps) {
         const int32_t p = __ldg(a.lrow + i);
@@ -308,12 +233,12 @@ __device__ void pull_long(const BfsArgs &a, Shared &s, const uint32_t *F, const 
         unsigned f = scan_row(a, F, st, head);
         if (f == kFull && head < en) {
             int q = 0;
-            if (lane == 0) q = atomicAdd(&s.nlist, 1);
+            if (lane == 0) q = atomicAdd(&s.rows.nlist, 1);
             q = __shfl_sync(kFull, q, 0);
             if (q < kPushRows) {
                 if (lane == 0) {
-                    s.list[q] = p;
-                    s.list_st[q] = i;
+                    s.rows.list[q] = p;
+                    s.rows.list_st[q] = i;
                 }
             } else {
                 f = scan_row(a, F, head, en);
@@ -327,9 +252,9 @@ __device__ void pull_long(const BfsArgs &a, Shared &s, const uint32_t *F, const 
         }
     }
     __syncthreads();
-    const int nrows = min(s.nlist, kPushRows);
+    const int nrows = min(s.rows.nlist, kPushRows);
     for (int q = 0; q < nrows; q++) {
-        const int i = s.list_st[q];
+        const int i = s.rows.list_st[q];
         const int64_t st = __ldg(a.lptr + i) + kLongChunk, en = __ldg(a.lptr + i + 1);
         if (threadIdx.x == 0) s.hit = kFull;
         __syncthreads();
@@ -349,7 +274,7 @@ __device__ void pull_long(const BfsArgs &a, Shared &s, const uint32_t *F, const 
         if (threadIdx.x == 0 && s.hit != kFull) {
             int32_t c = __ldg(a.lcol + st + s.hit);
             ALB_CHECK_ID(c, a.n, 0, &a.ctl->err);
-            a.parent_pos[s.list[q]] = (uint32_t)__ldg(a.perm + c);
+            a.parent_pos[s.rows.list[q]] = (uint32_t)__ldg(a.perm + c);
         }
         __syncthreads();
     }

@@ -67,9 +67,9 @@ struct List {
 struct Shared {
     BfsCtl c;
     // of the call: longest push row, rows and entries as GridArgs has them
-    int64_t max_out, m_in, m_out;
+    int64_t max_out, m_out;
     int level_cap, learned, cap;  // cap: of a list
-    int dir, form, lists, even, sparse, lean, ok, over, uneven;
+    int dir, form, lists, even, sparse, ok, over, uneven;
     Counts warp[kWarps];
     // sums of the last counting barrier; nbig: the big-row counter
     unsigned long long n, mo, mi, full, nbig;
@@ -693,15 +693,11 @@ __device__ void pull_long_tail(const BfsArgs &a, const uint32_t *F, unsigned lon
     }
 }
 
-// The group's first source in the frontier (-1: none). lean: the first column
-// alone is tested before the other three are fetched, which pays when most
-// columns hit (gathers of frontier words are what the pass is bound by).
+// The group's first source in the frontier (-1: none).
 template <bool kStaged>
-__device__ __forceinline__ int32_t test_group(const uint32_t *F, const int4 &c, bool lean) {
+__device__ __forceinline__ int32_t test_group(const uint32_t *F, const int4 &c) {
     auto word = [&](int32_t v) { return kStaged ? F[v >> 5] : __ldcg(F + (v >> 5)); };
-    const uint32_t f0 = word(c.x);
-    if (lean && ((f0 >> (c.x & 31)) & 1u)) return c.x;
-    const uint32_t f1 = word(c.y), f2 = word(c.z), f3 = word(c.w);
+    const uint32_t f0 = word(c.x), f1 = word(c.y), f2 = word(c.z), f3 = word(c.w);
     if ((f0 >> (c.x & 31)) & 1u) return c.x;
     if ((f1 >> (c.y & 31)) & 1u) return c.y;
     if ((f2 >> (c.z & 31)) & 1u) return c.z;
@@ -716,7 +712,7 @@ __device__ __forceinline__ int32_t test_group(const uint32_t *F, const int4 &c, 
 // quarter of the warps busy.
 template <bool kStaged>
 __device__ void pull_words(const BfsArgs &a, Shared &s, const uint32_t *F, uint32_t *N, int L,
-                           unsigned long long *ctr, bool lean) {
+                           unsigned long long *ctr) {
     constexpr int kW = 2;
     const int lane = lane_id();
     const int32_t C = a.C, log2C = a.log2C;
@@ -799,7 +795,7 @@ __device__ void pull_words(const BfsArgs &a, Shared &s, const uint32_t *F, uint3
                     ALB_CHECK_ID4(c[t], a.nwords * 32, p[t], &a.ctl->err);
                     // padding is the row itself, never in the frontier, and
                     // ends the row: the first hit is the smallest source
-                    found[t] = test_group<kStaged>(F, c[t], lean);
+                    found[t] = test_group<kStaged>(F, c[t]);
                     act[t] = found[t] < 0 && c[t].w != p[t];
                     c[t] = nx[t];
                 }
@@ -871,7 +867,7 @@ __device__ void pull_rows(const BfsArgs &a, Shared &s, uint16_t (*rows)[1024], c
                     for (int32_t j = 0; j < ng; j++) {
                         if (j) c = __ldcs(cp + (int64_t)j * C);
                         ALB_CHECK_ID4(c, a.nwords * 32, p, &a.ctl->err);
-                        found = test_group<false>(F, c, false);
+                        found = test_group<false>(F, c);
                         if (found >= 0 || c.w == p) break;
                     }
                 }
@@ -961,9 +957,10 @@ __device__ __forceinline__ void next_level(Shared &s, const BfsCtl &c) {
         s.even = even;
         s.lists = lists;
         s.nq[(c.level + 1) & 1] = 0;
-        // row shape: under ten unvisited rows in the words that have any
-        s.sparse = c.nu < 10 * c.active_words;
-        s.lean = c.mf > s.m_in / 4;
+        // row shape: under half of the rows of the words that have any unvisited
+        // (at 10 of 32 a uniform random graph of 2^24 takes 1,145 us, at 16 1,081;
+        // at 24 one of 2^22 364 -> 420)
+        s.sparse = c.nu < 16 * c.active_words;
     }
 }
 
@@ -1060,7 +1057,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_bfs_grid(BfsArgs a, InitParams 
     if (threadIdx.x == 0) {
         s.form = kQueue;
         s.max_out = x.max_out;
-        s.m_in = x.m_in;
         s.m_out = x.m_out;
         s.level_cap = in.level_cap;
         s.learned = learned;
@@ -1204,9 +1200,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_bfs_grid(BfsArgs a, InitParams 
                     pull_rows(a, s, pool.rows, F, N, L);
                 } else if (a.nwords * 4 <= kStageMax) {
                     if (!(ok = stage_frontier(a, s, pool.stage, F, staged++ & 1))) break;
-                    pull_words<true>(a, s, pool.stage, N, L, work, s.lean);
+                    pull_words<true>(a, s, pool.stage, N, L, work);
                 } else {
-                    pull_words<false>(a, s, F, N, L, work, s.lean);
+                    pull_words<false>(a, s, F, N, L, work);
                 }
                 next_form = kMap;
             }

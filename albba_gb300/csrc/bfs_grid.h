@@ -18,7 +18,7 @@ struct GridArgs {
     GridSlots *slots;
     const int4 *vrec;  // push rows' records, where list levels matter (row_recs_launch)
     int64_t max_out;  // longest push row (0: not known)
-    int64_t m_in, m_out;
+    int64_t m_out;
     int32_t sym;      // push and pull rows are the same
     BfsCtl *result;   // page-locked: level, done, err, levels_*, reached, edges
     int32_t list_cap;  // set by grid_launch

@@ -10,8 +10,14 @@
 // probes never leave the SM; the SELL-C-sigma and push-CSR arrays of each
 // graph stay in HBM, built by alb_sell_build with that graph's own C, sigma
 // and long-row threshold. Direction: Beamer alpha/beta per graph.
+// Bound: the largest items' own time, a chain of memory round trips per level
+// that a CTA can only spread over its warps: up to 1024 threads (at 64
+// registers, one CTA per SM) whatever fewer were asked for, pushes
+// dealt out evenly to threads (block_push), pulls two words per warp at a
+// time. 48 R-MAT graphs of 2^10 to 2^16 vertices, 8 roots each: 3.5 ms with
+// 256 threads, a row per warp and a word per warp at a time.
 // Output: level arrays (original ids), one per item, concatenated in the
-// order items were added. Graphs whose three bitmaps do not fit in one CTA's
+// order items were added. Graphs whose bitmaps do not fit in one CTA's
 // shared memory are not refused: their items run one by one on the
 // device-driven single-root path (alb_bfs_device, CUDA-graph level loop,
 // the entry's alpha and beta) into the same output, before the launch.
@@ -21,6 +27,7 @@
 #include <numeric>
 #include <vector>
 
+#include "block_push.cuh"
 #include "graph.h"
 
 namespace alb {
@@ -48,174 +55,267 @@ struct WlItem {
     int64_t out;  // offset of this item's level array
 };
 
-struct WlCounters {
-    unsigned long long n, mo, mi;
+constexpr int kPullWords = 2;  // words a warp pulls at a time
+
+struct WlShared {
+    int item, dir;
+    unsigned next_word;
+    unsigned n, mo, mi;  // what the level found
+    int nlong;           // long rows left after their head
+    int hit;
+    PushLists rows;      // list: those long rows' numbers
 };
 
-__global__ void k_worklist(const WlGraph *graphs, const WlItem *items, int32_t nitems,
-                           unsigned int *next_item, int32_t *out) {
-    extern __shared__ uint32_t sm[];
-    __shared__ int s_item;
-    __shared__ WlCounters s_acc;
-    const int lane = threadIdx.x & 31;
-    const int wib = threadIdx.x >> 5;
-    const int nw = blockDim.x >> 5;
+__device__ __forceinline__ void wl_count(WlShared &s, unsigned n, unsigned mo, unsigned mi) {
+    n = __reduce_add_sync(kFull, n);
+    mo = __reduce_add_sync(kFull, mo);
+    mi = __reduce_add_sync(kFull, mi);
+    if (lane_id() == 0 && n) {
+        atomicAdd(&s.n, n);
+        atomicAdd(&s.mo, mo);
+        atomicAdd(&s.mi, mi);
+    }
+}
+
+// Whether a source in [st, en) of the long-row list is in F (one warp).
+__device__ __forceinline__ bool wl_scan(const WlGraph &g, const uint32_t *F, int64_t st,
+                                        int64_t en) {
+    for (int64_t e0 = st + lane_id(); ; e0 += 128) {
+        bool hit = false;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int64_t e = e0 + 32 * u;
+            const int32_t c = e < en ? __ldg(g.lcol + e) : -1;
+            hit = hit || (c >= 0 && ((F[c >> 5] >> (c & 31)) & 1u));
+        }
+        if (__any_sync(kFull, hit)) return true;
+        if (__all_sync(kFull, e0 + 128 >= en)) return false;
+    }
+}
+
+// Unvisited long rows: a warp over the first kLongChunk sources of each, the
+// CTA together over the rest of a row without a source in the frontier there.
+template <int kT>
+__device__ void wl_pull_long(const WlGraph &g, WlShared &s, const uint32_t *F, const uint32_t *V,
+                             uint32_t *N, int32_t *lv, int L) {
+    const int lane = lane_id(), wib = threadIdx.x >> 5;
+    if (threadIdx.x == 0) s.nlong = 0;
+    __syncthreads();
+    unsigned n = 0, mo = 0, mi = 0;
+    auto reach = [&](int32_t p) {
+        atomicOr(&N[p >> 5], 1u << (p & 31));
+        lv[__ldg(g.perm + p)] = L + 1;
+        n++;
+        mo += (unsigned)__ldg(g.odeg + p);
+        mi += (unsigned)__ldg(g.ideg + p);
+    };
+    for (int64_t i = wib; i < g.nlong; i += kT / 32) {
+        const int32_t p = __ldg(g.lrow + i);
+        if ((V[p >> 5] >> (p & 31)) & 1u) continue;
+        const int64_t st = __ldg(g.lptr + i), en = __ldg(g.lptr + i + 1);
+        int64_t head = min(en, st + kLongChunk);
+        int q = 0;
+        bool found = wl_scan(g, F, st, head);
+        if (!found && head < en) {
+            if (lane == 0) q = atomicAdd(&s.nlong, 1);
+            q = __shfl_sync(kFull, q, 0);
+            if (q < kPushRows) {
+                if (lane == 0) s.rows.list[q] = (int32_t)i;
+            } else {  // (a full list: the warp scans the whole row)
+                found = wl_scan(g, F, head, en);
+            }
+        }
+        if (found && lane == 0) reach(p);
+    }
+    __syncthreads();
+    const int left = min(s.nlong, kPushRows);
+    for (int q = 0; q < left; q++) {
+        const int32_t i = s.rows.list[q];
+        const int64_t st = __ldg(g.lptr + i) + kLongChunk, en = __ldg(g.lptr + i + 1);
+        bool found = false;
+        for (int64_t e0 = st; e0 < en && !found; e0 += (kT / 32) * kLongChunk) {
+            const int64_t b = e0 + wib * kLongChunk;
+            found = __syncthreads_or(b < en && wl_scan(g, F, b, min(en, b + kLongChunk)));
+        }
+        if (found && threadIdx.x == 0) reach(__ldg(g.lrow + i));
+    }
+    wl_count(s, n, mo, mi);
+}
+
+// Bottom-up pull, kPullWords words per warp at a time, lane per row.
+__device__ __forceinline__ void wl_pull(const WlGraph &g, WlShared &s, const uint32_t *F,
+                                        const uint32_t *V, uint32_t *N, int32_t *lv, int L) {
+    const int lane = lane_id(), nw = (int)g.nwords;
+    unsigned n = 0, mo = 0, mi = 0;
     while (true) {
-        if (threadIdx.x == 0) s_item = (int)atomicAdd(next_item, 1u);
+        unsigned at = 0;
+        if (lane == 0) at = atomicAdd(&s.next_word, (unsigned)kPullWords);
+        const int wa = (int)__shfl_sync(kFull, at, 0);
+        if (wa >= nw) break;
+        int32_t p[kPullWords], ng[kPullWords];
+        bool act[kPullWords], found[kPullWords];
+        const int4 *cp[kPullWords];
+        int4 c[kPullWords];
+        int64_t so[kPullWords];
+#pragma unroll
+        for (int t = 0; t < kPullWords; t++) {
+            const uint32_t vis = wa + t < nw ? V[wa + t] : kFull;
+            p[t] = (wa + t) * 32 + lane;
+            act[t] = !((vis >> lane) & 1u);
+            found[t] = false;
+            const int32_t sl = (act[t] ? p[t] : 0) >> g.log2C;
+            ng[t] = act[t] ? (__ldg(g.width + sl) + 3) >> 2 : 0;
+            so[t] = act[t] ? __ldg(g.slice_off + sl) : 0;
+        }
+#pragma unroll
+        for (int t = 0; t < kPullWords; t++) {
+            cp[t] = g.col4 + (so[t] >> 2) + (p[t] & (g.C - 1));
+            c[t] = make_int4(p[t], p[t], p[t], p[t]);
+            if (ng[t] > 0) c[t] = __ldg(cp[t]);
+        }
+        for (int32_t j = 0;; j++) {
+            bool any = false;
+#pragma unroll
+            for (int t = 0; t < kPullWords; t++) {
+                act[t] = act[t] && j < ng[t];
+                any = any || act[t];
+            }
+            if (!__any_sync(kFull, any)) break;
+#pragma unroll
+            for (int t = 0; t < kPullWords; t++) {
+                if (!act[t]) continue;
+                int4 nx = make_int4(p[t], p[t], p[t], p[t]);
+                if (j + 1 < ng[t]) nx = __ldg(cp[t] + (int64_t)(j + 1) * g.C);
+                // (padding is the row itself, never in the frontier)
+                found[t] = ((F[c[t].x >> 5] >> (c[t].x & 31)) | (F[c[t].y >> 5] >> (c[t].y & 31)) |
+                            (F[c[t].z >> 5] >> (c[t].z & 31)) | (F[c[t].w >> 5] >> (c[t].w & 31))) & 1u;
+                act[t] = !found[t] && c[t].w != p[t];
+                c[t] = nx;
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < kPullWords; t++) {
+            if (wa + t >= nw) break;
+            const unsigned nm = __ballot_sync(kFull, found[t]);
+            if (lane == 0) N[wa + t] = nm;
+            if (found[t]) {
+                lv[__ldg(g.perm + p[t])] = L + 1;
+                n++;
+                mo += (unsigned)__ldg(g.odeg + p[t]);
+                mi += (unsigned)__ldg(g.ideg + p[t]);
+            }
+        }
+    }
+    wl_count(s, n, mo, mi);
+}
+
+// kT threads, 1024 / kT CTAs per SM.
+template <int kT>
+__global__ void __launch_bounds__(kT, 1024 / kT)
+    k_worklist(const WlGraph *graphs, const WlItem *items, int32_t nitems, unsigned int *next_item,
+               int32_t *out) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    WlShared &s = *reinterpret_cast<WlShared *>(smem);
+    uint32_t *maps = reinterpret_cast<uint32_t *>(smem + sizeof(WlShared));
+    const int lane = lane_id();
+    while (true) {
+        if (threadIdx.x == 0) s.item = (int)atomicAdd(next_item, 1u);
         __syncthreads();
-        const int it = s_item;
+        const int it = s.item;
         if (it >= nitems) break;
         const WlItem item = items[it];
         const WlGraph g = graphs[item.graph];
-        uint32_t *F = sm, *N = sm + g.nwords, *V = sm + 2 * g.nwords;
+        const int nw = (int)g.nwords;
+        uint32_t *F = maps, *N = maps + nw, *V = maps + 2 * nw;
         int32_t *lv = out + item.out;
-        for (int64_t w = threadIdx.x; w < g.nwords; w += blockDim.x) {
+        for (int w = threadIdx.x; w < nw; w += kT) {
             V[w] = g.vinit[w];
             F[w] = 0;
-            N[w] = 0;
         }
-        for (int64_t v = threadIdx.x; v < g.n; v += blockDim.x) lv[v] = -1;
+        for (int64_t v = threadIdx.x; v < g.n; v += kT) lv[v] = -1;
+        const int32_t rp = __ldg(g.inv + item.root);
+        unsigned nf = 1, prev_nf = 0, mf = (unsigned)__ldg(g.odeg + rp),
+                 mu = (unsigned)g.m_in - (unsigned)__ldg(g.ideg + rp);
         __syncthreads();
-        int64_t nf = 1, mf, prev_nf = 0, mu;
-        int prev_dir = -1;
         if (threadIdx.x == 0) {
-            const int32_t rp = g.inv[item.root];
             V[rp >> 5] |= 1u << (rp & 31);
             F[rp >> 5] |= 1u << (rp & 31);
             lv[item.root] = 0;
         }
-        {
-            const int32_t rp = g.inv[item.root];
-            mf = g.odeg[rp];
-            mu = g.m_in - g.ideg[rp];
-        }
+        int prev_dir = -1;
         __syncthreads();
         for (int L = 0; nf > 0 && L <= g.n; L++) {
-            // Beamer decision (identical in every thread)
-            int dir;
-            if (prev_dir < 0 || prev_dir == ALB_DIR_TOPDOWN)
-                dir = ((double)mf > (double)mu / g.alpha) ? ALB_DIR_BOTTOMUP : ALB_DIR_TOPDOWN;
-            else
-                dir = (nf >= prev_nf || (double)nf > (double)g.n / g.beta) ? ALB_DIR_BOTTOMUP
-                                                                           : ALB_DIR_TOPDOWN;
-            if (threadIdx.x == 0) s_acc.n = s_acc.mo = s_acc.mi = 0;
+            if (threadIdx.x == 0) {  // Beamer's rule (dev.cuh)
+                BfsCtl c;
+                c.prev_dir = prev_dir;
+                c.nf = nf;
+                c.prev_nf = prev_nf;
+                c.mf = mf;
+                c.mu = mu;
+                c.n = g.n;
+                c.alpha = g.alpha;
+                c.beta = g.beta;
+                s.dir = beamer_dir(c);
+                s.next_word = s.n = s.mo = s.mi = 0;
+            }
             __syncthreads();
-            unsigned long long cn = 0, cmo = 0, cmi = 0;
+            const int dir = s.dir;
             if (dir == ALB_DIR_BOTTOMUP) {
-                for (int64_t w = wib; w < g.nwords; w += nw) {
-                    const uint32_t vis = V[w];
-                    if (vis == kFull) {
-                        if (lane == 0) N[w] = 0;
-                        continue;
-                    }
-                    const int32_t p = (int32_t)(w * 32 + lane);
-                    bool active = !((vis >> lane) & 1u);
-                    int32_t ng = 0;
-                    const int4 *cp = nullptr;
-                    if (active) {
-                        const int64_t s = (int64_t)p >> g.log2C;
-                        ng = (__ldg(g.width + s) + 3) >> 2;
-                        cp = g.col4 + (__ldg(g.slice_off + s) >> 2) + (p & (g.C - 1));
-                    }
-                    bool found = false;
-                    for (int32_t j = 0;; j++) {
-                        active = active && j < ng;
-                        if (!__any_sync(kFull, active)) break;
-                        if (!active) continue;
-                        const int4 c = ld_nc(cp + (int64_t)j * g.C);
-                        const int32_t cc[4] = {c.x, c.y, c.z, c.w};
+                wl_pull(g, s, F, V, N, lv, L);
+                __syncthreads();
+                if (g.nlong) {
+                    wl_pull_long<kT>(g, s, F, V, N, lv, L);
+                    __syncthreads();
+                }
+                for (int w = threadIdx.x; w < nw; w += kT) V[w] |= N[w];
+            } else {
+                for (int w = threadIdx.x; w < nw; w += kT) N[w] = 0;
+                block_push<kT>(
+                    s.rows, F, 0, nw, kPushWords, g.pcol,
+                    [&](int32_t u, int32_t &st, int32_t &d, int32_t &ou) {
+                        st = (int32_t)__ldg(g.prow + u);
+                        d = (int32_t)__ldg(g.prow + u + 1) - st;
+                        ou = 0;
+                    },
+                    [&](const int32_t (&v)[4], const uint32_t (&)[4]) {
 #pragma unroll
                         for (int k = 0; k < 4; k++) {
-                            if (!active) break;
-                            if (cc[k] == p) {
-                                active = false;
-                            } else if ((F[cc[k] >> 5] >> (cc[k] & 31)) & 1u) {
-                                found = true;
-                                active = false;
-                            }
+                            if (v[k] < 0) continue;
+                            const uint32_t bit = 1u << (v[k] & 31);
+                            if ((V[v[k] >> 5] | N[v[k] >> 5]) & bit) continue;
+                            atomicOr(&N[v[k] >> 5], bit);
                         }
-                    }
-                    const unsigned nm = __ballot_sync(kFull, found);
-                    if (lane == 0) {
-                        N[w] = nm;
-                        V[w] = vis | nm;
-                    }
-                    if (found) {
-                        lv[__ldg(g.perm + p)] = L + 1;
-                        cn++;
-                        cmo += __ldg(g.odeg + p);
-                        cmi += __ldg(g.ideg + p);
-                    }
-                }
+                    });
                 __syncthreads();
-                // long rows: one warp each, frontier tests in shared memory
-                for (int64_t i = wib; i < g.nlong; i += nw) {
-                    const int32_t p = __ldg(g.lrow + i);
-                    const uint32_t bit = 1u << (p & 31);
-                    if (V[p >> 5] & bit) continue;
-                    const int64_t st = __ldg(g.lptr + i), en = __ldg(g.lptr + i + 1);
-                    bool found = false;
-                    for (int64_t e0 = st; e0 < en && !found; e0 += 32) {
-                        const int64_t e = e0 + lane;
-                        const int32_t c = e < en ? __ldg(g.lcol + e) : p;
-                        found = __any_sync(kFull, (F[c >> 5] >> (c & 31)) & 1u);
-                    }
-                    if (found && lane == 0) {
-                        atomicOr(&N[p >> 5], bit);
-                        atomicOr(&V[p >> 5], bit);
+                // the new frontier: levels, visited bits, counters; a warp per
+                // 32 words, lane per row
+                unsigned n = 0, mo = 0, mi = 0;
+                for (int wb = (int)(threadIdx.x & ~31u); wb < nw; wb += kT) {
+                    const uint32_t m = wb + lane < nw ? N[wb + lane] : 0u;
+                    if (m) V[wb + lane] |= m;
+                    for (unsigned todo = __ballot_sync(kFull, m != 0); todo; todo &= todo - 1) {
+                        const int q = __ffs(todo) - 1;
+                        if (!((__shfl_sync(kFull, m, q) >> lane) & 1u)) continue;
+                        const int32_t p = (wb + q) * 32 + lane;
                         lv[__ldg(g.perm + p)] = L + 1;
-                        cn++;
-                        cmo += __ldg(g.odeg + p);
-                        cmi += __ldg(g.ideg + p);
+                        n++;
+                        mo += (unsigned)__ldg(g.odeg + p);
+                        mi += (unsigned)__ldg(g.ideg + p);
                     }
                 }
-            } else {
-                // top-down: walk the set bits of F, one warp per frontier row
-                for (int64_t w = wib; w < g.nwords; w += nw) {
-                    uint32_t word = F[w];
-                    while (word) {
-                        const int b = __ffs(word) - 1;
-                        word &= word - 1;
-                        const int32_t u = (int32_t)(w * 32 + b);
-                        const int64_t st = __ldg(g.prow + u), en = __ldg(g.prow + u + 1);
-                        for (int64_t e = st + lane; e < en; e += 32) {
-                            const int32_t v = __ldg(g.pcol + e);
-                            const uint32_t bit = 1u << (v & 31);
-                            if (V[v >> 5] & bit) continue;
-                            if (!(atomicOr(&N[v >> 5], bit) & bit)) {
-                                lv[__ldg(g.perm + v)] = L + 1;
-                                cn++;
-                                cmo += __ldg(g.odeg + v);
-                                cmi += __ldg(g.ideg + v);
-                            }
-                        }
-                    }
-                }
-                __syncthreads();
-                for (int64_t w = threadIdx.x; w < g.nwords; w += blockDim.x) V[w] |= N[w];
-            }
-            cn = warp_sum(cn);
-            cmo = warp_sum(cmo);
-            cmi = warp_sum(cmi);
-            if (lane == 0 && cn) {
-                atomicAdd(&s_acc.n, cn);
-                atomicAdd(&s_acc.mo, cmo);
-                atomicAdd(&s_acc.mi, cmi);
+                wl_count(s, n, mo, mi);
             }
             __syncthreads();
-            // N becomes the frontier; the old frontier is cleared for reuse
-            uint32_t *t = F;
+            uint32_t *t = F;  // N becomes the frontier
             F = N;
             N = t;
-            for (int64_t w = threadIdx.x; w < g.nwords; w += blockDim.x) N[w] = 0;
             prev_nf = nf;
-            nf = (int64_t)s_acc.n;
-            mf = (int64_t)s_acc.mo;
-            mu -= (int64_t)s_acc.mi;
+            nf = s.n;
+            mf = s.mo;
+            mu -= s.mi;
             prev_dir = dir;
-            __syncthreads();
+            __syncthreads();  // the sums have been read
         }
-        __syncthreads();
     }
 }
 
@@ -284,10 +384,11 @@ alb_status alb_worklist_run_device(alb_worklist *w, int32_t block, int32_t *d_le
     ALB_CK(cudaSetDevice(g0->device));
     int max_smem = 0;
     ALB_CK(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, g0->device));
-    // a graph fits the kernel when its three bitmaps and 1 KB of other
-    // shared state fit in one CTA
+    // a graph fits the kernel when its three bitmaps and the rest of the
+    // shared state fit in one CTA (and its edges in 32-bit counters)
     auto fits = [&](const Sell &s) {
-        return sizeof(uint32_t) * 3 * (size_t)s.nwords + 1024 <= (size_t)max_smem;
+        return sizeof(uint32_t) * 3 * (size_t)s.nwords + sizeof(WlShared) + 1024 <= (size_t)max_smem &&
+               s.m_in <= INT32_MAX && s.m_out <= INT32_MAX;
     };
     std::vector<WlGraph> hg;
     std::vector<WlItem> hi;
@@ -356,7 +457,7 @@ alb_status alb_worklist_run_device(alb_worklist *w, int32_t block, int32_t *d_le
         }
         return ALB_OK;
     }
-    const size_t smem = sizeof(uint32_t) * 3 * (size_t)nwords_max;
+    const size_t smem = sizeof(WlShared) + sizeof(uint32_t) * 3 * (size_t)nwords_max;
     // longest items first
     std::vector<int32_t> order(hi.size());
     std::iota(order.begin(), order.end(), 0);
@@ -382,15 +483,23 @@ alb_status alb_worklist_run_device(alb_worklist *w, int32_t block, int32_t *d_le
         ALB_CK(cudaMemcpyAsync(di, sorted.data(), sizeof(WlItem) * sorted.size(),
                                cudaMemcpyHostToDevice, stream));
         ALB_CK(cudaMemsetAsync(dctr, 0, sizeof(unsigned int), stream));
-        ALB_CK(cudaFuncSetAttribute(k_worklist, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem));
+        // 1024 threads end the longest items soonest; where there are many
+        // items for every SM, two CTAs of 512 get more of them done; graphs of
+        // a word per warp of 256 threads and fewer than four have no use for more
+        const int threads = nwords_max <= 32 && block <= 256 ? 256
+                            : block == 1024 || (int64_t)sorted.size() <= 4 * (int64_t)g0->num_sms
+                                ? 1024
+                                : 512;
+        void (*f)(const WlGraph *, const WlItem *, int32_t, unsigned int *, int32_t *) =
+            threads == 256 ? k_worklist<256> : threads == 512 ? k_worklist<512> : k_worklist<1024>;
+        ALB_CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         int per_sm = 0;
-        ALB_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_worklist, block, smem));
+        ALB_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, threads, smem));
         if (per_sm < 1) return fail(ALB_ERR_UNSUPPORTED, "alb_worklist_run: kernel does not fit");
         const unsigned grid = (unsigned)std::min<int64_t>((int64_t)per_sm * g0->num_sms,
                                                           (int64_t)sorted.size());
         ALB_CK(cudaEventRecord(g0->ev0, stream));
-        k_worklist<<<grid, block, smem, stream>>>(dg, di, (int32_t)sorted.size(), dctr, d_levels);
+        f<<<grid, threads, smem, stream>>>(dg, di, (int32_t)sorted.size(), dctr, d_levels);
         ALB_CK(cudaGetLastError());
         ALB_CK(cudaEventRecord(g0->ev1, stream));
         ALB_CK(cudaStreamSynchronize(stream));
