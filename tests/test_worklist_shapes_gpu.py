@@ -58,3 +58,26 @@ def test_hubs_and_long_rows_1024_threads(opts):
 def test_largest_graph_that_fits():
     g = ab.gen_er(530_000, 6.0, seed=2)
     _run([(g, g.pick_roots(2, 1), (32, 1024, 1024))], 512)
+
+
+def test_frontiers_around_the_push_list_and_reuse_of_the_work_list():
+    """Top-down frontiers just under and over what the push lists at once (2,048
+    rows), spread over a large graph's words, and runs of one list one after
+    the other while items are added."""
+    n = 60_000
+    rng = np.random.default_rng(9)
+    wl, csrs = ab.Worklist(), []
+    for k in (2047, 2048, 2049, 5000):
+        # a star of k spokes with a leaf on each, ids shuffled
+        ids = rng.permutation(n)
+        spokes, leaves = ids[1:k + 1], ids[k + 1:2 * k + 1]
+        g = ab.csr_from_edges(n, np.concatenate([np.full(k, ids[0]), spokes]),
+                              np.concatenate([spokes, leaves]))
+        dg = ab.Graph(g)
+        dg.sell_build()
+        wl.add(dg, np.array([ids[0], leaves[0]], np.int32), alpha=1e-3)  # (top-down throughout)
+        csrs.append(g)
+        for _ in range(2):
+            levels, _ = wl.run(256)
+            for lv, (gi, root, _) in zip(levels, wl.layout):
+                assert np.array_equal(lv, oracle.bfs(csrs[gi].rowptr, csrs[gi].col, int(root))[0])
