@@ -22,6 +22,7 @@
 // device-driven single-root path (alb_bfs_device, the entry's alpha and beta) into the same output, before the launch.
 #include <algorithm>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <numeric>
 #include <vector>
@@ -332,6 +333,41 @@ struct alb_worklist {
     };
     std::vector<Entry> entries;
     int64_t total_out = 0;
+    // The launch's arguments: a page-locked image of the graphs, items and item
+    // counter, and its device copy. Filled anew by every run, kept between them
+    // (allocated and freed each time they cost 19 us); one run at a time.
+    std::mutex mu;
+    unsigned char *h_args = nullptr, *d_args = nullptr;
+    size_t args_cap = 0;
+    int device = 0;
+
+    // (on the current device, dev)
+    alb_status reserve(size_t bytes, int dev) {
+        if (bytes <= args_cap && dev == device) return ALB_OK;
+        release();
+        ALB_CK(cudaMallocHost((void **)&h_args, bytes));
+        const alb_status rc = alb::dmalloc((void **)&d_args, bytes, "worklist arguments");
+        if (rc != ALB_OK) {
+            release();
+            return rc;
+        }
+        args_cap = bytes;
+        device = dev;
+        return ALB_OK;
+    }
+    void release() {
+        if (!h_args) return;
+        int prev = -1;
+        cudaGetDevice(&prev);
+        cudaSetDevice(device);
+        cudaFreeHost(h_args);
+        alb::dfree(d_args);
+        cudaGetLastError();
+        if (prev >= 0) cudaSetDevice(prev);
+        h_args = d_args = nullptr;
+        args_cap = 0;
+    }
+    ~alb_worklist() { release(); }
 };
 
 using namespace alb;
@@ -467,24 +503,21 @@ alb_status alb_worklist_run_device(alb_worklist *w, int32_t block, int32_t *d_le
                      [&](int32_t a, int32_t b) { return cost[a] > cost[b]; });
     std::vector<WlItem> sorted(hi.size());
     for (size_t i = 0; i < order.size(); i++) sorted[i] = hi[order[i]];
-    WlGraph *dg = nullptr;
-    WlItem *di = nullptr;
-    unsigned int *dctr = nullptr;
-    auto cleanup = [&]() {
-        dfree(dg);
-        dfree(di);
-        dfree(dctr);
-    };
+    const size_t items_at = sizeof(WlGraph) * hg.size();
+    const size_t ctr_at = items_at + sizeof(WlItem) * sorted.size();
+    static_assert(sizeof(WlGraph) % 8 == 0 && sizeof(WlItem) % 8 == 0, "laid out one after the other");
+    const size_t args = ctr_at + 8;
+    std::lock_guard<std::mutex> lock(w->mu);
     alb_status rc = [&]() -> alb_status {
-        ALB_TRY(dmalloc((void **)&dg, sizeof(WlGraph) * hg.size(), "worklist graphs"));
-        ALB_TRY(dmalloc((void **)&di, sizeof(WlItem) * sorted.size(), "worklist items"));
-        ALB_TRY(dmalloc((void **)&dctr, sizeof(unsigned int), "worklist counter"));
+        ALB_TRY(w->reserve(args, g0->device));
+        std::memcpy(w->h_args, hg.data(), items_at);
+        std::memcpy(w->h_args + items_at, sorted.data(), ctr_at - items_at);
+        std::memset(w->h_args + ctr_at, 0, 8);
+        const WlGraph *dg = reinterpret_cast<const WlGraph *>(w->d_args);
+        const WlItem *di = reinterpret_cast<const WlItem *>(w->d_args + items_at);
+        unsigned int *dctr = reinterpret_cast<unsigned int *>(w->d_args + ctr_at);
         cudaStream_t stream = g0->stream;
-        ALB_CK(cudaMemcpyAsync(dg, hg.data(), sizeof(WlGraph) * hg.size(), cudaMemcpyHostToDevice,
-                               stream));
-        ALB_CK(cudaMemcpyAsync(di, sorted.data(), sizeof(WlItem) * sorted.size(),
-                               cudaMemcpyHostToDevice, stream));
-        ALB_CK(cudaMemsetAsync(dctr, 0, sizeof(unsigned int), stream));
+        ALB_CK(cudaMemcpyAsync(w->d_args, w->h_args, args, cudaMemcpyHostToDevice, stream));
         // 1024 threads end the longest items soonest; where there are many
         // items for every SM, two CTAs of 512 get more of them done; graphs of
         // a word per warp of 256 threads and fewer than four have no use for more
@@ -514,7 +547,7 @@ alb_status alb_worklist_run_device(alb_worklist *w, int32_t block, int32_t *d_le
         }
         return ALB_OK;
     }();
-    cleanup();
+    if (rc != ALB_OK) cudaStreamSynchronize(g0->stream);  // (the image may be on its way)
     return rc;
 }
 
