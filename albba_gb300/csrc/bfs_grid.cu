@@ -313,9 +313,29 @@ __device__ void map_to_list(const BfsArgs &a, const int4 *vrec, const List &q, i
     __syncthreads();
 }
 
-// The list back to the frontier bitmap F and, where Q is given, to the queue.
+// A row of d > kBigRow edges onto the grid-wide list, in chunks (push_big).
+__device__ __forceinline__ void put_big(const BfsArgs &a, unsigned long long *big_slot, int32_t u,
+                                        int64_t d) {
+    const unsigned long long nch = (unsigned long long)((d + kBigChunk - 1) / kBigChunk);
+    const unsigned long long old = atomicAdd(big_slot, (1ull << kBigShift) | nch);
+    const int64_t at = (int64_t)(old >> kBigShift);
+    a.big[at] = u;
+    a.big_base[at] = (int64_t)(old & kBigMask);
+}
+
+// The queue entry of row u where the big rows are listed as the queue is made:
+// those are in it as ~u, which push_rows passes over.
+__device__ __forceinline__ int32_t queued(const BfsArgs &a, unsigned long long *big_slot, int32_t u) {
+    const int32_t d = __ldg(a.odeg + u);
+    if (d <= kBigRow) return u;
+    put_big(a, big_slot, u, d);
+    return ~u;
+}
+
+// The list back to the frontier bitmap F and, where Q is given, to the queue
+// (big_slot, if given: big rows listed).
 __device__ void leave_list(const BfsArgs &a, Shared &s, const List &q, unsigned cnt, uint32_t *F,
-                           int32_t *Q, unsigned long long *q_slot) {
+                           int32_t *Q, unsigned long long *q_slot, unsigned long long *big_slot) {
     const int rows = (int)(cnt >> kRowShift);
     if (Q) {
         if (threadIdx.x == 0 && rows) s.at = atomicAdd(q_slot, (unsigned long long)rows);
@@ -324,7 +344,8 @@ __device__ void leave_list(const BfsArgs &a, Shared &s, const List &q, unsigned 
     for (int i = threadIdx.x; i < rows; i += kThreads) {
         const int32_t u = q.pos[i];
         if (F) atomicOr(F + (u >> 5), 1u << (u & 31));
-        if (Q && ALB_CHECK_POS(s.at + i, a.n, &a.ctl->err)) Q[s.at + i] = u;
+        if (Q && ALB_CHECK_POS(s.at + i, a.n, &a.ctl->err))
+            Q[s.at + i] = big_slot ? queued(a, big_slot, u) : u;
     }
 }
 
@@ -432,7 +453,7 @@ struct WarpRows {
 };
 
 // Rows of the queue, a few per warp, their edges flattened over the lanes;
-// rows longer than kBigRow go on a grid-wide list in chunks (push_big).
+// rows longer than kBigRow go on the grid-wide list if they are not on it.
 __device__ void push_rows(const BfsArgs &a, WarpRows *wr, const int32_t *Q, int64_t nf,
                           int64_t mf, uint32_t *N, unsigned long long *big_slot) {
     const int lane = lane_id(), wib = threadIdx.x >> 5;
@@ -449,16 +470,14 @@ __device__ void push_rows(const BfsArgs &a, WarpRows *wr, const int32_t *Q, int6
         int32_t ou = 0;
         if (lane < G && i < nf) {
             int32_t u = __ldcg(Q + i);
-            ALB_CHECK_ID(u, a.n, 0, &a.ctl->err);
-            st = __ldg(a.prow + u);
-            d = __ldg(a.prow + u + 1) - st;
-            ou = __ldg(a.perm + u);
+            if (u >= 0) {
+                ALB_CHECK_ID(u, a.n, 0, &a.ctl->err);
+                st = __ldg(a.prow + u);
+                d = __ldg(a.prow + u + 1) - st;
+                ou = __ldg(a.perm + u);
+            }
             if (d > kBigRow) {
-                const unsigned long long nch = (unsigned long long)((d + kBigChunk - 1) / kBigChunk);
-                const unsigned long long old = atomicAdd(big_slot, (1ull << kBigShift) | nch);
-                const int64_t at = (int64_t)(old >> kBigShift);
-                a.big[at] = u;
-                a.big_base[at] = (int64_t)(old & kBigMask);
+                put_big(a, big_slot, u, d);
                 d = 0;
             }
         }
@@ -550,7 +569,10 @@ __device__ void finish_push(const BfsArgs &a, Shared &s, uint16_t (*rows)[1024],
     const int lane = lane_id(), wib = threadIdx.x >> 5;
     const int64_t tid = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     const int64_t nth = (int64_t)gridDim.x * kThreads;
-    for (int64_t i = tid; i < nf; i += nth) F[__ldcg(Q + i) >> 5] = 0;
+    for (int64_t i = tid; i < nf; i += nth) {
+        const int32_t u = __ldcg(Q + i);
+        F[(u < 0 ? ~u : u) >> 5] = 0;
+    }
     unsigned cn = 0, full = 0;
     unsigned long long mo = 0, mi = 0;
     for (int64_t w0 = tid & ~31ll; w0 < a.nwords; w0 += nth) {
@@ -580,9 +602,10 @@ __device__ void finish_push(const BfsArgs &a, Shared &s, uint16_t (*rows)[1024],
     put_counts(s, cn, mo, mi, full);
 }
 
-// Frontier bitmap to queue, next bitmap cleared.
+// Frontier bitmap to queue (big rows listed), next bitmap cleared.
 __device__ void map_to_queue(const BfsArgs &a, uint16_t (*rows)[1024], const uint32_t *F,
-                             uint32_t *N, int32_t *Q, unsigned long long *q_slot) {
+                             uint32_t *N, int32_t *Q, unsigned long long *q_slot,
+                             unsigned long long *big_slot) {
     const int lane = lane_id(), wib = threadIdx.x >> 5;
     const int64_t tid = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     const int64_t nth = (int64_t)gridDim.x * kThreads;
@@ -600,7 +623,7 @@ __device__ void map_to_queue(const BfsArgs &a, uint16_t (*rows)[1024], const uin
         base = __shfl_sync(kFull, base, 0);
         for (int i = lane; i < tot; i += 32)
             if (ALB_CHECK_POS((int64_t)base + i, a.n, &a.ctl->err))
-                Q[base + i] = (int32_t)(w0 * 32) + rows[wib][i];
+                Q[base + i] = queued(a, big_slot, (int32_t)(w0 * 32) + rows[wib][i]);
         __syncwarp();
     }
 }
@@ -1115,7 +1138,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bfs_grid(BfsArgs a, InitParams 
         } else if (lists && (form == kQueue || even)) {
             const List q = list_at(pool, par, cap);
             if (even) {  // back to a queue first
-                leave_list(a, s, q, s.nq[par], F, Q, &a.ctl->qn[L % 3]);
+                leave_list(a, s, q, s.nq[par], F, Q, &a.ctl->qn[L % 3], nullptr);
                 form = kQueue;
                 if (!(ok = barrier(a, s, L))) break;
             }
@@ -1168,19 +1191,26 @@ __global__ void __launch_bounds__(kThreads, 1) k_bfs_grid(BfsArgs a, InitParams 
         } else {
             if (form == kList) {
                 leave_list(a, s, list_at(pool, par, cap), s.nq[par], F, dir == ALB_DIR_TOPDOWN ? Q : nullptr,
-                           &a.ctl->qn[L % 3]);
+                           &a.ctl->qn[L % 3], big);
                 count_active(a, s);
-                if (!(ok = barrier(a, s, L, acc + 4))) break;
+                if (!(ok = barrier(a, s, L, acc + 4, big))) break;
                 if (threadIdx.x == 0) s.c.active_words = (int64_t)s.n;
             }
             if (dir == ALB_DIR_TOPDOWN) {
                 if (form == kMap) {
-                    map_to_queue(a, pool.rows, F, N, Q, &a.ctl->qn[L % 3]);
-                    if (!(ok = barrier(a, s, L))) break;
+                    map_to_queue(a, pool.rows, F, N, Q, &a.ctl->qn[L % 3], big);
+                    if (!(ok = barrier(a, s, L, nullptr, big))) break;
                 }
+                // the big rows are known beforehand where the queue was made
+                // in this level: then they are pushed beside the others, a
+                // barrier and a phase of latency less (R-MAT 10^6: 28 -> 20 us).
+                // finish_push does not list them: most of its queues
+                // are of levels that turn out bottom-up.
+                const bool known = form != kQueue;
                 push_rows(a, wr, Q, nf, mf, N, big);
-                if (!(ok = barrier(a, s, L, nullptr, big))) break;
-                if (s.nbig) {
+                if (known && s.nbig) push_big(a, N, s.nbig);
+                if (!(ok = barrier(a, s, L, nullptr, known ? nullptr : big))) break;
+                if (!known && s.nbig) {
                     push_big(a, N, s.nbig);
                     if (!(ok = barrier(a, s, L))) break;
                 }

@@ -111,3 +111,26 @@ def test_directed_and_unaligned_outputs():
         assert np.array_equal(h[1:n + 1], olv) and np.array_equal(h[n + 2:2 * n + 2], opa)
         assert h[0] == h[n + 1] == h[-1] == 77
         assert dg.bfs_device(7).reached == int((olv >= 0).sum())
+
+
+@pytest.mark.parametrize("sizes", [(5000, 300, 257, 256, 255, 3), (257, 5000, 256, 1000, 258)])
+def test_big_rows_known_before_their_push(sizes):
+    """A chain of hubs either side of the length that is pushed in chunks
+    (256), reached from lists, queues and bottom-up levels' bitmaps."""
+    n = 20_011
+    ids = np.random.default_rng(4).permutation(n)
+    hubs, rest, u, v = ids[:len(sizes)], ids[len(sizes):], [], []
+    for i, k in enumerate(sizes):
+        u.append(np.full(k, hubs[i]))
+        v.append(rest[:k])
+        rest = rest[k:]
+    u.append(hubs[:-1])
+    v.append(hubs[1:])
+    g = ab.csr_from_edges(n, np.concatenate(u), np.concatenate(v))
+    with ab.Graph(g) as dg:
+        dg.sell_build()
+        for root in (hubs[0], hubs[-1], int(v[0][0])):
+            _check(g, dg, root, ab.bfs_opts("topdown"))
+            _check(g, dg, root, ab.bfs_opts("ref004"))
+            for alpha, beta in ((14.0, 24.0), (1e6, 0.5), (200.0, 2.0)):
+                _check(g, dg, root, ab.bfs_opts("beamer", alpha=alpha, beta=beta))
