@@ -561,11 +561,13 @@ __device__ __forceinline__ int list_bits(uint16_t *buf, uint32_t m) {
     return __shfl_sync(kFull, inc, 31);
 }
 
+// (sym, here and below: a row's two lengths are one number, loaded once: 1 to
+// 3 % of a search.)
 // After the pushes: the old frontier's bits are cleared over its queue, the
 // new frontier N goes to the next queue with levels, visited bits and counters.
 __device__ void finish_push(const BfsArgs &a, Shared &s, uint16_t (*rows)[1024], const int32_t *Q,
                             int64_t nf, uint32_t *F, const uint32_t *N, int32_t *NQ,
-                            unsigned long long *nq_slot, int L) {
+                            unsigned long long *nq_slot, int L, bool sym) {
     const int lane = lane_id(), wib = threadIdx.x >> 5;
     const int64_t tid = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     const int64_t nth = (int64_t)gridDim.x * kThreads;
@@ -592,7 +594,7 @@ __device__ void finish_push(const BfsArgs &a, Shared &s, uint16_t (*rows)[1024],
             const int32_t p = (int32_t)(w0 * 32) + rows[wib][i];
             if (ALB_CHECK_POS((int64_t)base + i, a.n, &a.ctl->err)) NQ[base + i] = p;
             a.level_pos[p] = L + 1;
-            const int32_t od = __ldg(a.odeg + p), id = __ldg(a.ideg + p);
+            const int32_t od = __ldg(a.odeg + p), id = sym ? od : __ldg(a.ideg + p);
             cn++;
             mo += (unsigned long long)od;
             mi += (unsigned long long)id;
@@ -735,7 +737,7 @@ __device__ __forceinline__ int32_t test_group(const uint32_t *F, const int4 &c) 
 // quarter of the warps busy.
 template <bool kStaged>
 __device__ void pull_words(const BfsArgs &a, Shared &s, const uint32_t *F, uint32_t *N, int L,
-                           unsigned long long *ctr) {
+                           unsigned long long *ctr, bool sym) {
     constexpr int kW = 2;
     const int lane = lane_id();
     const int32_t C = a.C, log2C = a.log2C;
@@ -841,7 +843,7 @@ __device__ void pull_words(const BfsArgs &a, Shared &s, const uint32_t *F, uint3
                 if (reached) {
                     a.level_pos[p[t]] = L + 1;
                     if (!by_long) a.parent_pos[p[t]] = (uint32_t)__ldg(a.perm + found[t]);
-                    const int32_t od = __ldg(a.odeg + p[t]), id = __ldg(a.ideg + p[t]);
+                    const int32_t od = __ldg(a.odeg + p[t]), id = sym ? od : __ldg(a.ideg + p[t]);
                     cn++;
                     mo += (unsigned long long)od;
                     mi += (unsigned long long)id;
@@ -854,7 +856,7 @@ __device__ void pull_words(const BfsArgs &a, Shared &s, const uint32_t *F, uint3
 
 // Row shape: the unvisited rows of 32 words, dealt out to the lanes.
 __device__ void pull_rows(const BfsArgs &a, Shared &s, uint16_t (*rows)[1024], const uint32_t *F,
-                          uint32_t *N, int L) {
+                          uint32_t *N, int L, bool sym) {
     const int lane = lane_id(), wib = threadIdx.x >> 5;
     const int32_t C = a.C, log2C = a.log2C;
     unsigned cn = 0, full = 0;
@@ -898,7 +900,7 @@ __device__ void pull_rows(const BfsArgs &a, Shared &s, uint16_t (*rows)[1024], c
                 if (reached) {
                     a.level_pos[p] = L + 1;
                     if (!by_long) a.parent_pos[p] = (uint32_t)__ldg(a.perm + found);
-                    const int32_t od = __ldg(a.odeg + p), id = __ldg(a.ideg + p);
+                    const int32_t od = __ldg(a.odeg + p), id = sym ? od : __ldg(a.ideg + p);
                     cn++;
                     mo += (unsigned long long)od;
                     mi += (unsigned long long)id;
@@ -1203,9 +1205,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_bfs_grid(BfsArgs a, InitParams 
                 }
                 // the big rows are known beforehand where the queue was made
                 // in this level: then they are pushed beside the others, a
-                // barrier and a phase of latency less (R-MAT 10^6: 28 -> 20 us).
-                // finish_push does not list them: most of its queues
-                // are of levels that turn out bottom-up.
+                // barrier and a phase of latency less (R-MAT of 10^6 vertices:
+                // 119 -> 114 us in all). finish_push does not list them: most
+                // of its queues are of levels that turn out bottom-up.
                 const bool known = form != kQueue;
                 push_rows(a, wr, Q, nf, mf, N, big);
                 if (known && s.nbig) push_big(a, N, s.nbig);
@@ -1214,7 +1216,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bfs_grid(BfsArgs a, InitParams 
                     push_big(a, N, s.nbig);
                     if (!(ok = barrier(a, s, L))) break;
                 }
-                finish_push(a, s, pool.rows, Q, nf, F, N, NQ, nqn, L);
+                finish_push(a, s, pool.rows, Q, nf, F, N, NQ, nqn, L, x.sym);
                 next_form = kQueue;
             } else {
                 if (long_left) {
@@ -1227,12 +1229,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_bfs_grid(BfsArgs a, InitParams 
                     }
                 }
                 if (s.sparse) {
-                    pull_rows(a, s, pool.rows, F, N, L);
+                    pull_rows(a, s, pool.rows, F, N, L, x.sym);
                 } else if (a.nwords * 4 <= kStageMax) {
                     if (!(ok = stage_frontier(a, s, pool.stage, F, staged++ & 1))) break;
-                    pull_words<true>(a, s, pool.stage, N, L, work);
+                    pull_words<true>(a, s, pool.stage, N, L, work, x.sym);
                 } else {
-                    pull_words<false>(a, s, F, N, L, work);
+                    pull_words<false>(a, s, F, N, L, work, x.sym);
                 }
                 next_form = kMap;
             }
