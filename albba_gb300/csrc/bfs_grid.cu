@@ -35,15 +35,20 @@ constexpr int kMaxBlocks = 160;     // fields of a list level's word
 constexpr int kCtl = kWarps - 1;    // the warp that waits at barriers and decides
 constexpr int kListThreads = kThreads - 32;  // the others hold a list's edges
 constexpr int kPer = 2;             // edges per thread and pass
-// A block's rows and edges at a list level: one pass, or two on graphs without
-// long rows (grids), whose searches are list levels almost throughout. More
-// shared memory would cost the other phases their L1.
-constexpr int kListCap = kPer * kListThreads, kListCapMax = 2 * kListCap;
+// A block's edges at a list level: one pass, or three on graphs without long
+// rows (grids), whose searches are list levels almost throughout. The grid of
+// 2^24 has frontiers of up to 150,000 rows and 570,000 edges: 12 to 15 us a
+// list level, 35 a level of queues (two passes were too few for 37 of its 503).
+constexpr int kListPass = kPer * kListThreads, kListCapMax = 3 * kListPass;
+// Its rows, which are what takes shared memory (and L1 from the other phases):
+// a claim past them goes to the queue and the bitmap (overflow).
+constexpr int kListRows = kListPass;
 constexpr int kFewEdges = 16;       // longest row of such a graph
 constexpr int kListRow = 255;       // the longest row that claims put on a list
-constexpr int kRowShift = 20;       // list counters: rows above, edges below
+constexpr int kRowShift = 19;       // list counters: rows above, edges below
 constexpr unsigned kEdgeMask = (1u << kRowShift) - 1;
-static_assert((int64_t)kListCapMax * kListRow <= kEdgeMask && kListCapMax < 1 << (32 - kRowShift),
+static_assert((int64_t)kListPass * kListRow <= kEdgeMask && kListCapMax * kFewEdges <= kEdgeMask &&
+                  kListCapMax < 1 << (32 - kRowShift),
               "a list's counter");
 constexpr int kBigShift = 38;  // big-row counter: rows above, chunks below
 constexpr unsigned long long kBigMask = (1ull << kBigShift) - 1;
@@ -58,7 +63,7 @@ struct __align__(16) Counts {
 };
 
 // A list's rows: start of the push row less the edges before it in the list,
-// those edges, the row's id and position. Four arrays of cap entries.
+// those edges, the row's id and position. Four arrays of kListRows entries.
 struct List {
     uint32_t *st;
     int32_t *off, *ou, *pos;
@@ -68,7 +73,7 @@ struct Shared {
     BfsCtl c;
     // of the call: longest push row, rows and entries as GridArgs has them
     int64_t max_out, m_out;
-    int level_cap, learned, cap;  // cap: of a list
+    int level_cap, learned, cap;  // cap: edges of a list
     int dir, form, lists, even, sparse, ok, over, uneven;
     Counts warp[kWarps];
     // sums of the last counting barrier; nbig: the big-row counter
@@ -83,7 +88,7 @@ struct Shared {
 // Dynamic shared memory: Shared, then one of these at a time: two lists by
 // level parity, the warps' row numbers, or the staged frontier.
 union Pool {
-    uint32_t lists[2 * 4 * kListCap];
+    uint32_t lists[2 * 4 * kListRows];
     uint16_t rows[kWarps][1024];  // bitmap bits of 32 words as row numbers
     uint32_t stage[1];
 };
@@ -95,9 +100,10 @@ constexpr size_t kPoolAt = (sizeof(Shared) + 15) & ~(size_t)15;
     Shared &s = *reinterpret_cast<Shared *>(dyn);        \
     Pool &pool = *reinterpret_cast<Pool *>(dyn + kPoolAt)
 
-__device__ __forceinline__ List list_at(Pool &pool, int par, int cap) {
-    uint32_t *b = pool.lists + (size_t)par * 4 * cap;
-    return List{b, (int32_t *)b + cap, (int32_t *)b + 2 * cap, (int32_t *)b + 3 * cap};
+__device__ __forceinline__ List list_at(Pool &pool, int par) {
+    constexpr int n = kListRows;
+    uint32_t *b = pool.lists + (size_t)par * 4 * n;
+    return List{b, (int32_t *)b + n, (int32_t *)b + 2 * n, (int32_t *)b + 3 * n};
 }
 
 // ------------------------------------------------------------- the barriers
@@ -188,11 +194,11 @@ __device__ bool barrier(const BfsArgs &a, Shared &s, int L, unsigned long long *
 // The list level's barrier word: 8 bits of arrivals, 8 of blocks whose next
 // list does not fit, 8 of blocks with more than five eighths of that, 20 of
 // claimed vertices, 20 of their edges, a block's counted up to 2^12 - 1: exact
-// while every list fits.
+// where neither flag is set.
 constexpr int kArrive = 56, kOver = 48, kUneven = 40, kVerts = 20, kEdgeBits = 12;
 static_assert(kMaxBlocks * kListCapMax < (1 << (kUneven - kVerts)) && kMaxBlocks < 256 &&
                   kMaxBlocks * ((1 << kEdgeBits) - 1) < (1 << kVerts) &&
-                  kListCapMax < (1 << kEdgeBits),
+                  5 * kListCapMax / 8 < (1 << kEdgeBits),
               "fields of the list word");
 
 // One warp, after the block's claims: arrives and waits, and leaves the sums in
@@ -204,7 +210,7 @@ __device__ __forceinline__ bool list_barrier(const BfsArgs &a, const GridArgs &x
                                              unsigned long long *word, unsigned long long *acc) {
     if (withheld(a, L)) return false;
     const unsigned mo = s.cmo, mi = s.cmi, cn = s.cn;
-    const bool over = s.wide || mo > (unsigned)s.cap;
+    const bool over = s.wide || mo > (unsigned)s.cap || cn > (unsigned)kListRows;
     const unsigned long long mine = (1ull << kArrive) | ((unsigned long long)over << kOver) |
                                     ((unsigned long long)(8 * mo > 5 * (unsigned)s.cap) << kUneven) |
                                     ((unsigned long long)cn << kVerts) |
@@ -228,13 +234,13 @@ __device__ __forceinline__ bool list_barrier(const BfsArgs &a, const GridArgs &x
         }
         v = ld_acquire(word);
     }
-    const bool any_over = ((v >> kOver) & 255) != 0;
+    const bool any_over = ((v >> kOver) & 255) != 0, any_uneven = ((v >> kUneven) & 255) != 0;
     unsigned long long emo = v & ((1u << kVerts) - 1);
-    if (any_over) emo = __ldcg(acc);
+    if (any_over || any_uneven) emo = __ldcg(acc);
     const unsigned long long emi = x.sym ? emo : __ldcg(acc + 1);
     if (lane == 0) {
         s.n = (v >> kVerts) & ((1u << (kUneven - kVerts)) - 1);
-        s.uneven = ((v >> kUneven) & 255) != 0;
+        s.uneven = any_uneven;
         s.over = any_over;
         s.mo = emo;
         s.mi = emi;
@@ -248,15 +254,17 @@ __device__ __forceinline__ bool list_barrier(const BfsArgs &a, const GridArgs &x
 
 // d_count: the row's edges as counted, at most kListRow where the list may
 // turn out too large to be used.
-__device__ __forceinline__ void append(const List &q, int cap, unsigned *nq, int32_t u, int64_t st,
+// False: no room.
+__device__ __forceinline__ bool append(const List &q, unsigned *nq, int32_t u, int64_t st,
                                        int32_t d_count, int32_t ou) {
     const unsigned at = atomicAdd(nq, (1u << kRowShift) | (unsigned)d_count);
     const unsigned i = at >> kRowShift, off = at & kEdgeMask;
-    if (i >= (unsigned)cap) return;  // (a queue's share that is then found not to fit)
+    if (i >= (unsigned)kListRows) return false;
     q.st[i] = (uint32_t)st - off;
     q.off[i] = (int32_t)off;
     q.ou[i] = ou;
     q.pos[i] = u;
+    return true;
 }
 
 // A push row's start, length and id: one 16-byte record (GridArgs::vrec), or
@@ -281,20 +289,21 @@ __device__ __forceinline__ RowRec row_rec(const BfsArgs &a, const int4 *vrec, in
 }
 
 __device__ __forceinline__ void append_row(const BfsArgs &a, const int4 *vrec, const List &q,
-                                           int cap, unsigned *nq, int32_t u, int32_t most) {
+                                           unsigned *nq, int32_t u, int32_t most) {
     ALB_CHECK_ID(u, a.n, 0, &a.ctl->err);
     const RowRec r = row_rec(a, vrec, u);
-    append(q, cap, nq, u, r.st, min(r.d, most), r.id);
+    // (no room: a queue's share that is then found not to fit)
+    append(q, nq, u, r.st, min(r.d, most), r.id);
 }
 
 // This block's share of the queue Q (nf rows) onto its list.
-__device__ void queue_to_list(const BfsArgs &a, const int4 *vrec, const List &q, int cap, unsigned *nq,
+__device__ void queue_to_list(const BfsArgs &a, const int4 *vrec, const List &q, unsigned *nq,
                               const int32_t *Q, int64_t nf, int32_t most) {
     if (threadIdx.x == 0) *nq = 0;
     __syncthreads();
     const int64_t b0 = nf * blockIdx.x / gridDim.x, b1 = nf * (blockIdx.x + 1) / gridDim.x;
     for (int64_t i = b0 + threadIdx.x; i < b1; i += kThreads)
-        append_row(a, vrec, q, cap, nq, __ldcg(Q + i), most);
+        append_row(a, vrec, q, nq, __ldcg(Q + i), most);
     __syncthreads();
 }
 
@@ -308,7 +317,7 @@ __device__ void map_to_list(const BfsArgs &a, const int4 *vrec, const List &q, i
         uint32_t m = __ldcg(F + w);
         N[w] = 0;
         if (m) F[w] = 0;
-        for (; m; m &= m - 1) append_row(a, vrec, q, cap, nq, (int32_t)(w * 32 + __ffs(m) - 1), cap);
+        for (; m; m &= m - 1) append_row(a, vrec, q, nq, (int32_t)(w * 32 + __ffs(m) - 1), cap);
     }
     __syncthreads();
 }
@@ -336,7 +345,7 @@ __device__ __forceinline__ int32_t queued(const BfsArgs &a, unsigned long long *
 // (big_slot, if given: big rows listed).
 __device__ void leave_list(const BfsArgs &a, Shared &s, const List &q, unsigned cnt, uint32_t *F,
                            int32_t *Q, unsigned long long *q_slot, unsigned long long *big_slot) {
-    const int rows = (int)(cnt >> kRowShift);
+    const int rows = min((int)(cnt >> kRowShift), kListRows);
     if (Q) {
         if (threadIdx.x == 0 && rows) s.at = atomicAdd(q_slot, (unsigned long long)rows);
         __syncthreads();
@@ -366,9 +375,10 @@ __device__ __forceinline__ void fetch_edges(const BfsArgs &a, const GridArgs &x,
     for (int k = 0; k < kPer; k++) {
         const int e = first + (int)threadIdx.x + k * kListThreads;
         E.v[k] = -1;
-        if (e >= ne || ne > cap || threadIdx.x >= kListThreads) continue;
+        if (e >= ne || ne > cap || nq > kListRows || threadIdx.x >= kListThreads) continue;
         int j = 0;  // the last row that starts at or before edge e
-        for (int step = 2048; step > 0; step >>= 1)
+        static_assert(kListRows <= 2048, "the first step");
+        for (int step = 1024; step > 0; step >>= 1)
             if (j + step < nq && q.off[j + step] <= e) j += step;
         E.v[k] = __ldg(a.pcol + (uint32_t)(q.st[j] + (uint32_t)e));
         ALB_CHECK_ID(E.v[k], a.n, -1, &a.ctl->err);
@@ -377,6 +387,16 @@ __device__ __forceinline__ void fetch_edges(const BfsArgs &a, const GridArgs &x,
 #pragma unroll
     for (int k = 0; k < kPer; k++)
         if (E.v[k] >= 0) E.r[k] = row_rec(a, x.vrec, E.v[k]);
+}
+
+// A claim of level L without room in the block's next list (which is then
+// taken for over, and left): its place in the next queue and bitmap at once.
+__device__ __noinline__ void overflow(const BfsArgs &a, int32_t v, int L) {
+    uint32_t *N = (L & 1) ? a.bm0 : a.bm1;
+    int32_t *NQ = (L & 1) ? a.q0 : a.q1;
+    const unsigned long long at = atomicAdd(&a.ctl->qn[(L + 1) % 3], 1ull);
+    if (ALB_CHECK_POS(at, a.n, &a.ctl->err)) NQ[at] = v;
+    atomicOr(N + (v >> 5), 1u << (v & 31));
 }
 
 // Targets are claimed by the compare-and-swap that moves their level from -1.
@@ -395,7 +415,8 @@ __device__ __forceinline__ void list_level(const BfsArgs &a, const GridArgs &x, 
         atomicMin(a.parent_pos + E.v[k], E.ou[k]);
         if (was[k] != -1) continue;
         atomicOr(a.vis + (E.v[k] >> 5), 1u << (E.v[k] & 31));
-        append(nx, s.cap, nnx, E.v[k], E.r[k].st, min(E.r[k].d, kListRow), E.r[k].id);
+        if (!append(nx, nnx, E.v[k], E.r[k].st, min(E.r[k].d, kListRow), E.r[k].id))
+            overflow(a, E.v[k], L);
         if (E.r[k].d > kListRow) s.wide = 1;
         n++;
         mo += (unsigned)E.r[k].d;
@@ -965,15 +986,16 @@ __device__ __forceinline__ void next_level(Shared &s, const BfsCtl &c) {
     } else {
         dir = rule_dir(c);
     }
-    // lists: no block may hold more rows or edges than s.cap. From lists, the
+    // lists: no block may hold more than kListRows rows or s.cap edges. From lists, the
     // last barrier said whether one does; from a queue or bitmap, the whole
     // frontier fits one block, or (queue) its equal shares should fit with
     // room to spare, which is checked once they are laid out -- as when lists
     // that grew apart are dealt out anew.
     const int64_t nb = gridDim.x;
     const bool listed = s.form == kList;
-    const bool all_fit = c.mf <= s.cap && c.nf <= s.cap;
-    const bool shares = s.max_out <= kListRow && 4 * c.mf <= 3 * s.cap * nb;
+    const bool all_fit = c.mf <= s.cap && c.nf <= kListRows;
+    const bool shares = s.max_out <= kListRow && 4 * c.mf <= 3 * s.cap * nb &&
+                        4 * c.nf <= 3 * kListRows * nb;
     const bool td = dir == ALB_DIR_TOPDOWN && s.m_out <= UINT32_MAX && s.max_out < (1 << 20);
     const bool even = listed && shares && (s.over || (s.uneven && 2 * c.mf <= s.cap * nb));
     const bool lists = td && (listed ? !s.over || even : all_fit || (s.form == kQueue && shares));
@@ -1136,19 +1158,19 @@ __global__ void __launch_bounds__(kThreads, 1) k_bfs_grid(BfsArgs a, InitParams 
         const int par = L & 1;
         int next_form;
         if (lists && form == kMap) {
-            map_to_list(a, x.vrec, list_at(pool, par, cap), cap, &s.nq[par], F, N);
+            map_to_list(a, x.vrec, list_at(pool, par), cap, &s.nq[par], F, N);
         } else if (lists && (form == kQueue || even)) {
-            const List q = list_at(pool, par, cap);
+            const List q = list_at(pool, par);
             if (even) {  // back to a queue first
                 leave_list(a, s, q, s.nq[par], F, Q, &a.ctl->qn[L % 3], nullptr);
                 form = kQueue;
                 if (!(ok = barrier(a, s, L))) break;
             }
-            const bool all = mf <= cap && nf <= cap;
-            queue_to_list(a, x.vrec, q, cap, &s.nq[par], Q, nf, all ? cap : kListRow);
+            const bool all = mf <= cap && nf <= kListRows;
+            queue_to_list(a, x.vrec, q, &s.nq[par], Q, nf, all ? cap : kListRow);
             const unsigned k = s.nq[par];
             if (!all) {  // does every block's share fit?
-                const bool no = (k & kEdgeMask) > (unsigned)cap || (k >> kRowShift) > (unsigned)cap;
+                const bool no = (k & kEdgeMask) > (unsigned)cap || (k >> kRowShift) > (unsigned)kListRows;
                 put_counts(s, threadIdx.x == 0 && no, 0, 0, 0);
                 if (!(ok = barrier(a, s, L, acc + 8))) break;
                 lists = s.n == 0;
@@ -1162,13 +1184,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_bfs_grid(BfsArgs a, InitParams 
             // list levels until another form is due; while the control warp
             // waits and decides, the others fetch the next level's edges
             Edges E;
-            fetch_edges(a, x, list_at(pool, par, cap), cap, s.nq[par], 0, E);
+            fetch_edges(a, x, list_at(pool, par), cap, s.nq[par], 0, E);
             for (int l = L;;) {
                 const int p = l & 1;
-                const List cur = list_at(pool, p, cap), nx = list_at(pool, p ^ 1, cap);
+                const List cur = list_at(pool, p), nx = list_at(pool, p ^ 1);
                 const unsigned cnt = s.nq[p];
                 list_level(a, x, s, E, nx, &s.nq[p ^ 1], l);
-                for (int e = kListCap; e < (int)(cnt & kEdgeMask); e += kListCap) {
+                for (int e = kListPass; e < (int)(cnt & kEdgeMask); e += kListPass) {
                     fetch_edges(a, x, cur, cap, cnt, e, E);
                     list_level(a, x, s, E, nx, &s.nq[p ^ 1], l);
                 }
@@ -1192,7 +1214,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bfs_grid(BfsArgs a, InitParams 
             continue;
         } else {
             if (form == kList) {
-                leave_list(a, s, list_at(pool, par, cap), s.nq[par], F, dir == ALB_DIR_TOPDOWN ? Q : nullptr,
+                leave_list(a, s, list_at(pool, par), s.nq[par], F, dir == ALB_DIR_TOPDOWN ? Q : nullptr,
                            &a.ctl->qn[L % 3], big);
                 count_active(a, s);
                 if (!(ok = barrier(a, s, L, acc + 4, big))) break;
@@ -1310,9 +1332,9 @@ __global__ void __launch_bounds__(kScatterThreads)
     }
 }
 
-size_t shared_bytes(int64_t nwords, int list_cap) {
+size_t shared_bytes(int64_t nwords) {
     const int64_t stage = nwords * 4 <= kStageMax ? (nwords * 4 + 15) & ~15ll : 0;
-    return kPoolAt + std::max({sizeof(Pool), (size_t)stage, sizeof(uint32_t) * 8 * (size_t)list_cap});
+    return kPoolAt + std::max(sizeof(Pool), (size_t)stage);
 }
 
 }  // namespace
@@ -1325,10 +1347,10 @@ bool grid_takes(const alb_graph *g, const alb_bfs_opts &o, const BfsArgs &a) {
 alb_status grid_launch(const alb_graph *g, const BfsArgs &a, const InitParams &in,
                        const GridArgs &args_in, cudaStream_t st) {
     GridArgs x = args_in;
-    x.list_cap = x.max_out <= kFewEdges ? kListCapMax : kListCap;
-    const size_t smem = shared_bytes(a.nwords, x.list_cap);
+    x.list_cap = x.max_out <= kFewEdges ? kListCapMax : kListPass;
+    const size_t smem = shared_bytes(a.nwords);
     ALB_CK(cudaFuncSetAttribute(k_bfs_grid, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)shared_bytes(kStageMax / 4, kListCapMax)));
+                                (int)shared_bytes(kStageMax / 4)));
     BfsArgs aa = a;
     InitParams ii = in;
     GridArgs xx = x;

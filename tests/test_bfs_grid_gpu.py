@@ -134,3 +134,19 @@ def test_big_rows_known_before_their_push(sizes):
             _check(g, dg, root, ab.bfs_opts("ref004"))
             for alpha, beta in ((14.0, 24.0), (1e6, 0.5), (200.0, 2.0)):
                 _check(g, dg, root, ab.bfs_opts("beamer", alpha=alpha, beta=beta))
+
+
+@pytest.mark.parametrize("arity,depth", [(2, 17), (3, 11), (15, 4), (15, 5)])
+def test_claims_past_a_lists_rows(arity, depth):
+    """Trees: a block's list of up to 5,952 edges (rows of at most 16) claims as
+    many rows, three times what the next list has room for."""
+    n = (arity ** (depth + 1) - 1) // (arity - 1)
+    child = np.arange(1, n)
+    ids = np.random.default_rng(6).permutation(n)
+    for perm in (np.arange(n), ids):
+        g = ab.csr_from_edges(n, perm[(child - 1) // arity], perm[child])
+        with ab.Graph(g) as dg:
+            dg.sell_build()
+            for root in (perm[0], perm[1], perm[n - 1]):
+                for policy in ("topdown", "beamer", "learned", "ref004"):
+                    _check(g, dg, root, ab.bfs_opts(policy, "persistent"))
