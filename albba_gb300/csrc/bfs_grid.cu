@@ -400,12 +400,15 @@ __device__ __noinline__ void overflow(const BfsArgs &a, int32_t v, int L) {
 }
 
 // Targets are claimed by the compare-and-swap that moves their level from -1.
-__device__ __forceinline__ void list_level(const BfsArgs &a, const GridArgs &x, Shared &s,
-                                           const Edges &E, const List &nx, unsigned *nnx, int L) {
-    int32_t was[kPer];
+__device__ __forceinline__ void claim(const BfsArgs &a, const Edges &E, int L, int32_t (&was)[kPer]) {
 #pragma unroll
     for (int k = 0; k < kPer; k++)
         was[k] = E.v[k] >= 0 ? atomicCAS(a.level_pos + E.v[k], -1, L + 1) : 0;
+}
+
+__device__ __forceinline__ void list_level(const BfsArgs &a, const GridArgs &x, Shared &s,
+                                           const Edges &E, const int32_t (&was)[kPer],
+                                           const List &nx, unsigned *nnx, int L) {
     unsigned n = 0, mo = 0, mi = 0;
 #pragma unroll
     for (int k = 0; k < kPer; k++) {
@@ -1189,10 +1192,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_bfs_grid(BfsArgs a, InitParams 
                 const int p = l & 1;
                 const List cur = list_at(pool, p), nx = list_at(pool, p ^ 1);
                 const unsigned cnt = s.nq[p];
-                list_level(a, x, s, E, nx, &s.nq[p ^ 1], l);
-                for (int e = kListPass; e < (int)(cnt & kEdgeMask); e += kListPass) {
-                    fetch_edges(a, x, cur, cap, cnt, e, E);
-                    list_level(a, x, s, E, nx, &s.nq[p ^ 1], l);
+                for (int e = 0;;) {
+                    int32_t was[kPer];
+                    claim(a, E, l, was);
+                    const Edges now = E;
+                    e += kListPass;
+                    const bool more = e < (int)(cnt & kEdgeMask);
+                    if (more) fetch_edges(a, x, cur, cap, cnt, e, E);
+                    list_level(a, x, s, now, was, nx, &s.nq[p ^ 1], l);
+                    if (!more) break;
                 }
                 __syncthreads();
                 if (ctl) {
