@@ -89,8 +89,11 @@ struct MsArgs {
     int32_t *q0, *q1;
     int32_t *big;  // frontier rows longer than kBigRow (top-down)
     int64_t *big_base;
+    int32_t *pbig;  // the same of the pushed roots' rows: the long rows' list is in use
+    int64_t *pbig_base;
     MsCtl *ctl;
     MsSample *smp;  // directly after *ctl
+    int32_t any_big;   // some push row is longer than kBigRow
     int32_t long_row;  // rows with more sources than this are the long rows
     const float *mlp;
     long long *gtrace;  // kGTraceCap x kGTraceW level records (MsCtl::gtrace_on)
@@ -189,21 +192,23 @@ __device__ __forceinline__ void ms_start(const MsArgs &a, const MsInit &in, int6
 // than `split` are left to ms_pull_wide. Call from all lanes of a warp.
 template <bool kSkip>
 struct MsWords {
-    int64_t cur, nxt;     // first word of the current run and of the next one
+    int32_t cur, nxt;     // first word of the current run and of the next one
     uint32_t dcur, dnxt;  // lane l < step: done word of word cur + l / nxt + l
     unsigned left;        // words of the current run not yet yielded
     unsigned ncur, nnxt;  // words of the runs that are not left out
     int step, split;
-    __device__ __forceinline__ int64_t grab(const MsStep &x, unsigned long long *ctr) const {
+    // (words past the last are taken for a.nwords)
+    __device__ __forceinline__ int32_t grab(const MsArgs &a, const MsStep &x,
+                                            unsigned long long *ctr) const {
         unsigned long long v = 0;
         if ((threadIdx.x & 31) == 0) v = atomicAdd(ctr, (unsigned long long)step);
-        return x.nwarps * step + (int64_t)__shfl_sync(kFull, v, 0);
+        return (int32_t)min(a.nwords, x.nwarps * step + (int64_t)__shfl_sync(kFull, v, 0));
     }
-    __device__ __forceinline__ void load(const MsArgs &a, int64_t r, uint32_t &d, unsigned &n) const {
+    __device__ __forceinline__ void load(const MsArgs &a, int32_t r, uint32_t &d, unsigned &n) const {
         const int l = threadIdx.x & 31;
         bool mine = l < step && r + l < a.nwords;
         d = mine ? a.D[r + l] : kFull;
-        if (mine && split != INT32_MAX) mine = __ldg(a.width + (((r + l) * 32) >> a.log2C)) <= split;
+        if (mine && split != INT32_MAX) mine = __ldg(a.width + (((int64_t)(r + l) * 32) >> a.log2C)) <= split;
         n = __ballot_sync(kFull, mine);
     }
     __device__ __forceinline__ unsigned prep(uint64_t *N, uint32_t *An) const {
@@ -212,7 +217,7 @@ struct MsWords {
         const unsigned full = __ballot_sync(kFull, dcur == kFull) & ncur;
         for (unsigned f = full; f; f &= f - 1) {
             const int q = __ffs(f) - 1;
-            N[(cur + q) * 32 + l] = 0;
+            N[(int64_t)(cur + q) * 32 + l] = 0;
             if (l == 0) An[cur + q] = 0;
         }
         return ncur & ~full;
@@ -221,26 +226,26 @@ struct MsWords {
                                           unsigned long long *ctr) {
         step = run;
         split = wide;
-        cur = x.gw * step;
-        nxt = grab(x, ctr);
+        cur = (int32_t)min(a.nwords, x.gw * step);
+        nxt = grab(a, x, ctr);
         load(a, cur, dcur, ncur);
         load(a, nxt, dnxt, nnxt);
         left = prep(x.N, x.An);
     }
     // the next word (a.nwords when the level's words are exhausted) and its
     // done word
-    __device__ __forceinline__ int64_t next(const MsArgs &a, const MsStep &x,
+    __device__ __forceinline__ int32_t next(const MsArgs &a, const MsStep &x,
                                             unsigned long long *ctr, uint32_t &d) {
         while (!left) {
             if (cur >= a.nwords) {
                 d = kFull;
-                return a.nwords;
+                return (int32_t)a.nwords;
             }
             cur = nxt;
             dcur = dnxt;
             ncur = nnxt;
             if (cur < a.nwords) {
-                nxt = grab(x, ctr);
+                nxt = grab(a, x, ctr);
                 load(a, nxt, dnxt, nnxt);
             }
             left = prep(x.N, x.An);
@@ -316,12 +321,12 @@ __device__ __forceinline__ void ms_pull(const MsArgs &a, const MsStep &x, int ru
     // overlaps the current word's column loads and gathers.
     MsWords<kBypass> it;
     it.start(a, x, run, split, ctr);
-    auto geometry = [&](int64_t ww, uint32_t dd, uint64_t &vv, int32_t &wdv, int64_t &sov) {
+    auto geometry = [&](int32_t ww, uint32_t dd, uint64_t &vv, int32_t &wdv, int64_t &sov) {
         vv = kAll;
         wdv = 0;
         sov = 0;
         if (ww < a.nwords && !(kBypass && dd == kFull)) {
-            const int64_t pw = ww * 32 + lane;
+            const int64_t pw = (int64_t)ww * 32 + lane;
             // rows past n (padding of the last word) are preset visited;
             // their slice index is clamped so the loads stay in bounds
             const int64_t sw = (pw < a.n ? pw : a.n - 1) >> a.log2C;
@@ -331,18 +336,19 @@ __device__ __forceinline__ void ms_pull(const MsArgs &a, const MsStep &x, int ru
         }
     };
     uint32_t d, d1 = kFull;
-    int64_t w = it.next(a, x, ctr, d);
-    int64_t w1 = w < a.nwords ? it.next(a, x, ctr, d1) : a.nwords;
+    const int32_t nwords = (int32_t)a.nwords;
+    int32_t w = it.next(a, x, ctr, d);
+    int32_t w1 = w < nwords ? it.next(a, x, ctr, d1) : nwords;
     uint64_t vis_c;
     int32_t wd_c;
     int64_t so_c;
     geometry(w, d, vis_c, wd_c, so_c);
-    while (w < a.nwords) {
+    while (w < nwords) {
         uint64_t vis1;
         int32_t wd1;
         int64_t so1;
         geometry(w1, d1, vis1, wd1, so1);
-        const int64_t p = w * 32 + lane;
+        const int64_t p = (int64_t)w * 32 + lane;
         if (kBypass && d == kFull) {  // not reached: MsWords clears these words
             N[p] = 0;
             if (lane == 0) An[w] = 0;
@@ -418,7 +424,7 @@ __device__ __forceinline__ void ms_pull(const MsArgs &a, const MsStep &x, int ru
         vis_c = vis1;
         wd_c = wd1;
         so_c = so1;
-        w1 = w1 < a.nwords ? it.next(a, x, ctr, d1) : a.nwords;
+        w1 = w1 < nwords ? it.next(a, x, ctr, d1) : nwords;
     }
     cnt.bytes += bytes;
 }
@@ -743,6 +749,29 @@ __device__ __forceinline__ void ms_push4(const MsArgs &a, uint64_t *N, uint32_t 
     }
 }
 
+// A row of d > kBigRow edges onto the list that all warps share (ms_push_big).
+template <bool kPush>
+__device__ __forceinline__ void ms_put_big(const MsArgs &a, unsigned long long *big_slot, int32_t u,
+                                           int64_t d) {
+    const unsigned long long nch = (unsigned long long)((d + kBigChunk - 1) / kBigChunk);
+    const unsigned long long old = atomicAdd(big_slot, (1ull << kMsBigShift) | nch);
+    const int64_t idx = (int64_t)(old >> kMsBigShift);
+    (kPush ? a.pbig : a.big)[idx] = u;
+    (kPush ? a.pbig_base : a.big_base)[idx] = (int64_t)(old & kMsBigMask);
+}
+
+// Row u's entry in a queue made at the level that pushes it: a big row is
+// listed at once and stands in the queue as ~u, which ms_push_rows passes over,
+// so that both kinds can be pushed in one step.
+template <bool kPush>
+__device__ __forceinline__ int32_t ms_queued(const MsArgs &a, unsigned long long *big_slot, int32_t u) {
+    if (!a.any_big) return u;
+    const int32_t d = __ldg(a.odeg + u);
+    if (d <= kBigRow) return u;
+    ms_put_big<kPush>(a, big_slot, u, d);
+    return ~u;
+}
+
 // Top-down push over the frontier queue. kPush: the push of a bottom-up
 // level's tmask roots, over the queue ms_tq built (next-parity queue and
 // counters, which that level leaves unused), with the state updated in place.
@@ -768,12 +797,8 @@ __device__ __forceinline__ void ms_push_rows(const MsArgs &a, const MsStep &x,
             d = __ldg(a.prow + u + 1) - st;
             f = ms_ld(F + u) & tm;
             if (kPush) cnt.bytes += 20;  // queue entry, row offsets, frontier word
-            if (d > kBigRow) {  // pushed in chunks by all warps in ms_push_big
-                const unsigned long long nch = (unsigned long long)((d + kBigChunk - 1) / kBigChunk);
-                const unsigned long long old = atomicAdd(big_slot, (1ull << kMsBigShift) | nch);
-                const int64_t idx = (int64_t)(old >> kMsBigShift);
-                a.big[idx] = u;
-                a.big_base[idx] = (int64_t)(old & kMsBigMask);
+            if (d > kBigRow) {  // pushed in chunks by all warps
+                ms_put_big<kPush>(a, big_slot, u, d);
                 d = 0;
             }
         }
@@ -813,6 +838,8 @@ template <bool kPush>
 __device__ __forceinline__ void ms_push_big(const MsArgs &a, const MsStep &x,
                                             unsigned long long ctr, MsCounts &cnt) {
     const uint64_t tm = kPush ? x.tm : kAll;
+    const int32_t *big = kPush ? a.pbig : a.big;
+    const int64_t *big_base = kPush ? a.pbig_base : a.big_base;
     const int64_t nbig = (int64_t)(ctr >> kMsBigShift);
     const int64_t total = (int64_t)(ctr & kMsBigMask);
     const uint64_t *F = x.F;
@@ -823,20 +850,20 @@ __device__ __forceinline__ void ms_push_big(const MsArgs &a, const MsStep &x,
     int64_t lo = 0, hi = nbig - 1;
     while (lo < hi) {
         const int64_t mid = (lo + hi + 1) >> 1;
-        if (a.big_base[mid] <= k0) lo = mid;
+        if (big_base[mid] <= k0) lo = mid;
         else hi = mid - 1;
     }
-    int64_t base = a.big_base[lo];
-    int64_t next = lo + 1 < nbig ? a.big_base[lo + 1] : total;
-    int32_t u = a.big[lo];
+    int64_t base = big_base[lo];
+    int64_t next = lo + 1 < nbig ? big_base[lo + 1] : total;
+    int32_t u = big[lo];
     int64_t st = __ldg(a.prow + u), d = __ldg(a.prow + u + 1) - st;
     uint64_t f = ms_ld(F + u) & tm;
     for (int64_t k = k0; k < k1; k++) {
         while (k >= next) {  // the run crosses into the next long row
             lo++;
             base = next;
-            next = lo + 1 < nbig ? a.big_base[lo + 1] : total;
-            u = a.big[lo];
+            next = lo + 1 < nbig ? big_base[lo + 1] : total;
+            u = big[lo];
             st = __ldg(a.prow + u);
             d = __ldg(a.prow + u + 1) - st;
             f = ms_ld(F + u) & tm;
@@ -892,9 +919,10 @@ __device__ __forceinline__ int ms_words_at_once(const MsArgs &a, const MsStep &x
 }
 
 // Frontier-nonzero bitmap Az -> queue, before a top-down level that follows a
-// bottom-up one (or none).
+// bottom-up one (or none). Big rows are listed (big_slot).
 __device__ __forceinline__ void ms_compact(const MsArgs &a, const MsStep &x, int32_t *Q,
-                                           unsigned long long *qslot) {
+                                           unsigned long long *qslot,
+                                           unsigned long long *big_slot) {
     const int lane = threadIdx.x & 31, per = ms_words_at_once(a, x);
     for (int64_t w0 = x.gw * per; w0 < a.nwords; w0 += x.nwarps * per) {
         const int64_t w = w0 + lane;
@@ -907,7 +935,7 @@ __device__ __forceinline__ void ms_compact(const MsArgs &a, const MsStep &x, int
         if (lane == 31) base = atomicAdd(qslot, (unsigned long long)total);
         base = __shfl_sync(kFull, base, 31);
         int64_t o = (int64_t)base + inc - cnt;
-        for (; m; m &= m - 1) Q[o++] = (int32_t)(w * 32 + __ffs(m) - 1);
+        for (; m; m &= m - 1) Q[o++] = ms_queued<false>(a, big_slot, (int32_t)(w * 32 + __ffs(m) - 1));
     }
 }
 
@@ -966,10 +994,11 @@ __device__ __forceinline__ void ms_finish(const MsArgs &a, const MsStep &x, uint
 }
 
 // Queue of the rows in the level's frontier that hold a tmask root, for the
-// push after a bottom-up level's pull. A warp takes 32 bitmap words at a time
-// and reads the frontier words of the set bits only.
+// push after a bottom-up level's pull, big rows listed. A warp takes 32 bitmap
+// words at a time and reads the frontier words of the set bits only.
 __device__ __forceinline__ void ms_tq(const MsArgs &a, const MsStep &x, int32_t *Q,
-                                      unsigned long long *qslot, MsCounts &c) {
+                                      unsigned long long *qslot, unsigned long long *big_slot,
+                                      MsCounts &c) {
     const int lane = threadIdx.x & 31, per = ms_words_at_once(a, x);
     for (int64_t w0 = x.gw * per; w0 < a.nwords; w0 += x.nwarps * per) {
         const uint32_t mine = lane < per && w0 + lane < a.nwords ? ms_ld(x.Az + w0 + lane) : 0u;
@@ -991,7 +1020,7 @@ __device__ __forceinline__ void ms_tq(const MsArgs &a, const MsStep &x, int32_t 
         int64_t o = (int64_t)base + inc - __popc(hits);
         c.bytes += 4 * __popc(hits);  // queue entries
         for (; hits; hits &= hits - 1)
-            Q[o++] = (int32_t)((w0 + lane) * 32 + __ffs(hits) - 1);
+            Q[o++] = ms_queued<true>(a, big_slot, (int32_t)((w0 + lane) * 32 + __ffs(hits) - 1));
     }
 }
 

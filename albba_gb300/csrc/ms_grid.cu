@@ -6,10 +6,10 @@
 // to 10 kernels behind a switch and a while node, about 43 us on R-MAT scale
 // 16 whatever the level held. Here a level takes one barrier (a pull) to five
 // (a push with long rows and samples), some 1.5 us each, and steps without
-// work are not run. 37 roots on R-MAT scale 16, search and output: 418 -> 182
-// us; 64 on scale 20: 690 -> 440; 64 on scale 24: 3,565 -> 3,403, of which the
+// work are not run. 37 roots on R-MAT scale 16, search and output: 418 -> 175
+// us; 64 on scale 20: 690 -> 409; 64 on scale 24: 3,565 -> 3,340, of which the
 // two large pulls (970 and 400) are bound by their gathers, one address per
-// clock and SM, and the output (970) by memory.
+// clock and SM, and the output (870) by memory.
 //
 // The block keeps under 8 KB of shared memory: L1 holds the gathers' hubs.
 // With 40 KB (the selector's weights and a frontier row table copied there)
@@ -31,7 +31,7 @@ using Level = MsSlots::Level;
 struct Shared {
     MsCtl c;
     MsSums sum;               // the level's sums at the last counting barrier
-    unsigned long long word;  // the counter that the last barrier read
+    unsigned long long word[2];  // the counters that the last barrier read
     MsSums warp[kWarps];
     unsigned long long room[128];
     int ok;
@@ -80,7 +80,7 @@ __device__ __forceinline__ void put(Shared &s, const MsCounts &c) {
 // Grid barrier on the arrival counter, which is never reset: a block's barrier
 // ends when the count reaches the next multiple of the block count. acc (null:
 // none): every warp's sums are added up there and read back into s.sum. word
-// (null: none): read into s.word.
+// (null: none): two counters read into s.word.
 __device__ bool barrier(const MsArgs &a, const MsGridArgs &x, Shared &s, int L,
                         MsSums *acc = nullptr, const unsigned long long *word = nullptr) {
     if (x.withhold_level >= 0 && L == x.withhold_level && (int)blockIdx.x == x.withhold_block)
@@ -129,7 +129,8 @@ __device__ bool barrier(const MsArgs &a, const MsGridArgs &x, Shared &s, int L,
         if (lane == 0) s.ok = ok && !(v & kBarFailed);
         __syncwarp();
         if (acc && lane < kSums) reinterpret_cast<unsigned long long *>(&s.sum)[lane] = __ldcg(sums + lane);
-        if (word && lane == kSums) s.word = __ldcg(word);
+        if (word && lane >= kSums && lane < kSums + 2)
+            s.word[lane - kSums] = __ldcg(word + lane - kSums);
     }
     __syncthreads();
     return s.ok;
@@ -241,14 +242,18 @@ __device__ __forceinline__ bool level_down(const MsArgs &a, const MsGridArgs &x,
     const int wib = threadIdx.x >> 5;
     int32_t *Q = (p.L & 1) ? a.q1 : a.q0;
     MsCounts cnt;
-    if (!s.c.q_valid) ms_compact(a, p, Q, &l.qn);
+    // a queue made here has its big rows listed: they are pushed beside the
+    // others (R-MAT scale 16: level 0 24 -> 18 us)
+    const bool known = !s.c.q_valid;
+    if (known) ms_compact(a, p, Q, &l.qn, &l.nbig);
     ms_zero_next(a, p);
-    if (!barrier(a, x, s, p.L, nullptr, &l.qn)) return false;
-    if (blockIdx.x == 0 && threadIdx.x < 64) a.smp->deg[threadIdx.x] = 0;
-    ms_push_rows<false>(a, p, Q, (int64_t)s.word, &l.nbig, cnt);
     if (!barrier(a, x, s, p.L, nullptr, &l.nbig)) return false;
-    if (s.word) {
-        ms_push_big<false>(a, p, s.word, cnt);
+    if (blockIdx.x == 0 && threadIdx.x < 64) a.smp->deg[threadIdx.x] = 0;
+    ms_push_rows<false>(a, p, Q, (int64_t)s.word[1], &l.nbig, cnt);
+    if (known && s.word[0]) ms_push_big<false>(a, p, s.word[0], cnt);
+    if (!barrier(a, x, s, p.L, nullptr, known ? nullptr : &l.nbig)) return false;
+    if (!known && s.word[0]) {
+        ms_push_big<false>(a, p, s.word[0], cnt);
         if (!barrier(a, x, s, p.L)) return false;
     }
     ms_finish(a, p, s.buf[wib], (p.L & 1) ? a.q0 : a.q1, &next.qn, cnt);
@@ -267,7 +272,7 @@ __device__ __forceinline__ bool long_rows(const MsArgs &a, const MsGridArgs &x, 
     ms_long_head<kEarly>(a, p, filt, &l.nbig, cnt);
     put(s, cnt);
     if (!barrier(a, x, s, p.L, &l.acc, &l.nbig)) return false;
-    const unsigned long long ctr = s.word;
+    const unsigned long long ctr = s.word[0];
     if (!ctr) return true;
     MsCounts tail;
     ms_long_tail<kEarly>(a, p, filt, ctr, tail);
@@ -280,12 +285,15 @@ __device__ __forceinline__ bool long_rows(const MsArgs &a, const MsGridArgs &x, 
 // A bottom-up level up to its counts. False: a wait gave up.
 __device__ __forceinline__ bool level_up(const MsArgs &a, const MsGridArgs &x, Shared &s,
                                          const MsStep &p, Level &l) {
-    const int wib = threadIdx.x >> 5;
     int32_t *Q = (p.L & 1) ? a.q0 : a.q1;  // (the next level's: idle here)
     const bool early = s.c.dir == ALB_DIR_BOTTOMUP;
+    if (p.tm) {
+        MsCounts cnt;
+        ms_tq(a, p, Q, &l.pqn, &l.pbig, cnt);
+        put(s, cnt);
+    }
     {
         MsCounts cnt;
-        if (p.tm) ms_tq(a, p, Q, &l.pqn, cnt);
         if (early) {
             // wide words by teams where runs are short, that is where a level is
             // not many times a wide word's time: at the first bottom-up level
@@ -302,21 +310,15 @@ __device__ __forceinline__ bool level_up(const MsArgs &a, const MsGridArgs &x, S
         }
         put(s, cnt);
     }
-    if (!barrier(a, x, s, p.L, &l.acc, &l.pqn)) return false;
-    const int64_t pq = (int64_t)s.word;
+    if (!barrier(a, x, s, p.L, &l.acc, &l.pbig)) return false;
+    const unsigned long long big = s.word[0];
+    const int64_t pq = (int64_t)s.word[1];
     if (a.nlong && !(early ? long_rows<true>(a, x, s, p, l) : long_rows<false>(a, x, s, p, l)))
         return false;
     if (!pq) return true;
-    {
-        MsCounts cnt;
-        ms_push_rows<true>(a, p, Q, pq, &l.pbig, cnt);
-        put(s, cnt);
-    }
-    if (!barrier(a, x, s, p.L, &l.acc, &l.pbig)) return false;
-    const unsigned long long big = s.word;
-    if (!big) return true;
     MsCounts cnt;
-    ms_push_big<true>(a, p, big, cnt);
+    ms_push_rows<true>(a, p, Q, pq, &l.pbig, cnt);
+    if (big) ms_push_big<true>(a, p, big, cnt);
     put(s, cnt);
     return barrier(a, x, s, p.L, &l.acc);
 }

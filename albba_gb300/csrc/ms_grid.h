@@ -13,9 +13,9 @@ struct MsSlots {
     unsigned long long bar, pad[15];
     struct Level {
         MsSums acc;
-        // long-row and long-frontier-row counter, queue length, word counter,
-        // and the pushed roots' queue length and long-row counter
-        unsigned long long nbig, qn, work, pqn, pbig, pad[3];
+        // long-row and long-frontier-row counter, queue length; the pushed
+        // roots' long-row counter and queue length; word counter
+        unsigned long long nbig, qn, pbig, pqn, work, pad[3];
     } level[4];
 };
 

@@ -172,7 +172,7 @@ __global__ void k_ms_bu_long_fin(MsArgs a, int j) {
 // The queue of the running level's frontier.
 __global__ void k_ms_compact(MsArgs a, int j) {
     const MsStep x = ms_step(a, j);
-    ms_compact(a, x, (x.L & 1) ? a.q1 : a.q0, &a.ctl->qn[x.L % 3]);
+    ms_compact(a, x, (x.L & 1) ? a.q1 : a.q0, &a.ctl->qn[x.L % 3], &a.ctl->nbig[x.L % 3]);
 }
 
 __global__ void k_ms_zero_next(MsArgs a, int j) { ms_zero_next(a, ms_step(a, j)); }
@@ -223,7 +223,8 @@ __global__ void k_ms_tq(MsArgs a, int j) {
     const MsStep x = ms_step(a, j);
     if (!x.tm) return;
     MsCounts cnt;
-    ms_tq(a, x, ((x.L + 1) & 1) ? a.q1 : a.q0, &a.ctl->qn[(x.L + 1) % 3], cnt);
+    ms_tq(a, x, ((x.L + 1) & 1) ? a.q1 : a.q0, &a.ctl->qn[(x.L + 1) % 3],
+          &a.ctl->nbig[(x.L + 1) % 3], cnt);
     ms_count(a, x.L, cnt);
 }
 
@@ -467,6 +468,8 @@ struct MsScratch {
     uint32_t *D = nullptr, *A = nullptr;
     int32_t *q0 = nullptr, *q1 = nullptr, *big = nullptr;
     int64_t *big_base = nullptr;
+    int32_t *pbig = nullptr;
+    int64_t *pbig_base = nullptr;
     MsCtl *ctl = nullptr, *h_ctl = nullptr;
     int32_t *out = nullptr;
     long long *gtrace = nullptr;  // the cooperative kernel's level records
@@ -494,6 +497,8 @@ void ms_scratch_free(alb_graph *g) {
     dfree(m.q1);
     dfree(m.big);
     dfree(m.big_base);
+    dfree(m.pbig);
+    dfree(m.pbig_base);
     dfree(m.ctl);
     dfree(m.out);
     dfree(m.gtrace);
@@ -559,6 +564,10 @@ alb_status ms_alloc(alb_graph *g, MsScratch &m) {
     ALB_TRY(dmalloc((void **)&m.q1, sizeof(int32_t) * npad, "msbfs queue"));
     ALB_TRY(dmalloc((void **)&m.big, sizeof(int32_t) * npad, "msbfs long-row list"));
     ALB_TRY(dmalloc((void **)&m.big_base, sizeof(int64_t) * npad, "msbfs long-row chunk bases"));
+    // (rows of more than kBigRow edges: there cannot be more)
+    const size_t nbig = (size_t)std::min<int64_t>(npad, s.m_out / kBigRow + 1);
+    ALB_TRY(dmalloc((void **)&m.pbig, sizeof(int32_t) * nbig, "msbfs pushed rows"));
+    ALB_TRY(dmalloc((void **)&m.pbig_base, sizeof(int64_t) * nbig, "msbfs pushed rows' chunk bases"));
     ALB_TRY(dmalloc((void **)&m.ctl, sizeof(MsCtl) + sizeof(MsSample), "msbfs control"));
     ALB_TRY(dmalloc((void **)&m.gtrace, sizeof(long long) * kGTraceCap * kGTraceW,
                     "msbfs level records"));
@@ -593,6 +602,7 @@ MsArgs ms_args(alb_graph *g, MsScratch &m) {
     a.pcol = s.pcol;
     a.nlong = s.nlong;
     a.long_row = s.long_row;
+    a.any_big = s.max_deg > kBigRow;
     a.lrow = s.lrow;
     a.lptr = s.lptr;
     a.lcol = s.lcol;
@@ -604,6 +614,8 @@ MsArgs ms_args(alb_graph *g, MsScratch &m) {
     a.q1 = m.q1;
     a.big = m.big;
     a.big_base = m.big_base;
+    a.pbig = m.pbig;
+    a.pbig_base = m.pbig_base;
     a.ctl = m.ctl;
     a.smp = reinterpret_cast<MsSample *>(m.ctl + 1);
     a.gtrace = m.gtrace;
