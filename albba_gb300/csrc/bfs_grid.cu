@@ -756,41 +756,48 @@ __device__ __forceinline__ int32_t test_group(const uint32_t *F, const int4 &c) 
 
 // Word shape: a warp takes runs of words from the level's counter, lane l's
 // visited word loaded a run ahead, and pulls two words at a time, lane per
-// row. run: words per run, a quarter of what an even split gives a warp (32 at
-// most): with runs of 32 whatever the size, a graph of 2^20 vertices kept a
-// quarter of the warps busy.
+// row. Runs shrink towards the level's end, from a quarter of what an even
+// split gives a warp (32 words at most) to 4: with equal runs of 26 words half
+// of the warps of R-MAT scale 24 had nothing left for the last fifth of the
+// level. A uniform random graph of 2^24 1,025 -> 975 us in all, R-MAT of
+// 2^23 255 -> 243, scale 24 from a leaf 379 -> 367 and from a hub 614 -> 610;
+// equal runs of 8: 985, 248, 381, 643. Bound: the gathers of frontier bits, an
+// address per clock and SM (2^22 vertices of mean degree 8: 31 M in 108 us).
 template <bool kStaged>
 __device__ void pull_words(const BfsArgs &a, Shared &s, const uint32_t *F, uint32_t *N, int L,
                            unsigned long long *ctr, bool sym) {
     constexpr int kW = 2;
     const int lane = lane_id();
     const int32_t C = a.C, log2C = a.log2C;
-    const int run = (int)min((int64_t)32, max((int64_t)kW, a.nwords / ((int64_t)gridDim.x * kWarps * 4)));
+    const int64_t warps = (int64_t)gridDim.x * kWarps;
+    const int most = (int)min((int64_t)32, max((int64_t)kW, a.nwords / (warps * 4))), least = min(4, most);
+    int64_t nxt = 0;
+    int run = 0;  // words of the run at nxt
     const uint64_t pol = l2_evict_first();
     unsigned cn = 0, full = 0;
     unsigned long long mo = 0, mi = 0;
+    // the next run, and its visited words
     auto grab = [&]() {
+        run = max(least, (int)min((int64_t)most, (a.nwords - nxt) / (warps * 6)));
         unsigned long long v = 0;
         if (lane == 0) v = atomicAdd(ctr, (unsigned long long)run);
-        return (int64_t)__shfl_sync(kFull, v, 0);
+        nxt = (int64_t)__shfl_sync(kFull, v, 0);
+        return lane < run && nxt + lane < a.nwords ? __ldcg(a.vis + nxt + lane) : kFull;
     };
-    auto run_vis = [&](int64_t rw) {
-        return lane < run && rw + lane < a.nwords ? __ldcg(a.vis + rw + lane) : kFull;
-    };
-    int64_t cur = grab(), nxt = grab();
-    uint32_t vcur = run_vis(cur), vnxt = run_vis(nxt);
+    uint32_t vcur = grab();
+    int64_t cur = nxt;
+    int rcur = run;
+    uint32_t vnxt = grab();
     while (cur < a.nwords) {
-        const bool valid = lane < run && cur + lane < a.nwords;
+        const bool valid = lane < rcur && cur + lane < a.nwords;
         if (valid && vcur == kFull) N[cur + lane] = 0;
         unsigned todo = __ballot_sync(kFull, valid && vcur != kFull);
         const int64_t base_w = cur;
         const uint32_t vrun = vcur;
         cur = nxt;
         vcur = vnxt;
-        if (cur < a.nwords) {
-            nxt = grab();
-            vnxt = run_vis(nxt);
-        }
+        rcur = run;
+        if (cur < a.nwords) vnxt = grab();
         while (todo) {
             int qs[kW], nr = 0;
 #pragma unroll
