@@ -118,7 +118,12 @@ struct MsCounts {
     unsigned long long mo = 0, mi = 0, edges = 0, bytes = 0;
 };
 
-// One level as a step sees it, and the calling warp's place in the launch.
+// One level as a step sees it, and the calling warp's place in the launch:
+// the first warps of all blocks come first, so that work for fewer warps than
+// there are is spread over all SMs (64 K vertices have 2,048 words for 4,864
+// warps), and each next one turned by five blocks, so that every 4th, 16th or
+// 32nd piece of work -- a sort window's widest rows -- is not always the same
+// blocks' (152 SMs; the first pull of 2^22 took 633 us instead of 532).
 struct MsStep {
     int L;
     const uint64_t *F;   // this level's frontier and the next one's
@@ -127,12 +132,15 @@ struct MsStep {
     uint32_t *An;
     uint64_t tm;         // roots that are pushed at a bottom-up level
     int64_t gw, nwarps;
+    bool numbered;  // the pull's first runs by warp number, not from the counter
 };
 
-__device__ __forceinline__ MsStep ms_step(const MsArgs &a, int L, int j, uint64_t tm) {
+__device__ __forceinline__ MsStep ms_step(const MsArgs &a, int L, int j, uint64_t tm,
+                                          bool numbered) {
+    const unsigned wib = threadIdx.x >> 5;
     return MsStep{L, slot(a, j), slot(a, j + 1), nz_bits(a, L), nz_bits(a, L + 1), tm,
-                  (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5),
-                  (int64_t)gridDim.x * (blockDim.x >> 5)};
+                  (int64_t)wib * gridDim.x + (blockIdx.x + 5 * wib) % gridDim.x,
+                  (int64_t)gridDim.x * (blockDim.x >> 5), numbered};
 }
 
 // The control block before level 0, from what the roots came to.
@@ -182,9 +190,9 @@ __device__ __forceinline__ void ms_start(const MsArgs &a, const MsInit &in, int6
 }
 
 // Words of a bottom-up level in runs of `run` words (1 to 32, set by the
-// host from the word count: about three runs per warp): a warp's first run by
-// its number, the others from the level's counter (dynamic distribution, as
-// WordRuns). The done words of a run are loaded together, one per lane, a run
+// host from the word count: about three runs per warp) from the level's
+// counter (dynamic distribution, as WordRuns); where x.numbered is set a warp's
+// first run goes by its number, which saves a round trip. The done words of a run are loaded together, one per lane, a run
 // ahead of use. kSkip: words whose rows are all done are not yielded; their
 // next-frontier words and nonzero bits are cleared when the run comes up, one
 // coalesced store per word, so a warp does not walk them one dependent round
@@ -202,7 +210,8 @@ struct MsWords {
                                             unsigned long long *ctr) const {
         unsigned long long v = 0;
         if ((threadIdx.x & 31) == 0) v = atomicAdd(ctr, (unsigned long long)step);
-        return (int32_t)min(a.nwords, x.nwarps * step + (int64_t)__shfl_sync(kFull, v, 0));
+        return (int32_t)min(a.nwords, (x.numbered ? x.nwarps * step : 0) +
+                                          (int64_t)__shfl_sync(kFull, v, 0));
     }
     __device__ __forceinline__ void load(const MsArgs &a, int32_t r, uint32_t &d, unsigned &n) const {
         const int l = threadIdx.x & 31;
@@ -226,7 +235,7 @@ struct MsWords {
                                           unsigned long long *ctr) {
         step = run;
         split = wide;
-        cur = (int32_t)min(a.nwords, x.gw * step);
+        cur = x.numbered ? (int32_t)min(a.nwords, x.gw * step) : grab(a, x, ctr);
         nxt = grab(a, x, ctr);
         load(a, cur, dcur, ncur);
         load(a, nxt, dnxt, nnxt);
@@ -447,7 +456,7 @@ __device__ __forceinline__ void ms_pull_wide(const MsArgs &a, const MsStep &x, i
                                              uint64_t *room, MsCounts &cnt) {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int team = wib / kTeam, k = wib % kTeam;
-    const int64_t teams = x.nwarps / kTeam, t = x.gw / kTeam;
+    const int64_t teams = x.nwarps / kTeam, t = (int64_t)team * gridDim.x + blockIdx.x;
     const int64_t all = (int64_t)a.nwin * a.wpw;
     unsigned *acc_lo = reinterpret_cast<unsigned *>(room + team * 32) + 2 * lane, *acc_hi = acc_lo + 1;
     for (int64_t i0 = t; i0 < all; i0 += 32 * teams) {

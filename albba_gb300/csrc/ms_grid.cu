@@ -356,7 +356,7 @@ k_ms_grid(const __grid_constant__ MsArgs a, const __grid_constant__ MsInit in,
     while (ok && !s.c.done) {
         const int L = s.c.level;
         Level &l = x.slots->level[L % 3], &next = x.slots->level[(L + 1) % 3];
-        const MsStep p = ms_step(a, L, L - s.c.base, s.c.tmask);
+        const MsStep p = ms_step(a, L, L - s.c.base, s.c.tmask, true);
         long long *rec = first && s.c.gtrace_on && L < kGTraceCap ? a.gtrace + (int64_t)L * kGTraceW : nullptr;
         if (rec) rec[0] = (long long)globaltimer_ns();
         // the next level's counters: read last at level L - 2, and every block

@@ -42,7 +42,7 @@ constexpr uint64_t kMsBarrierNs = 4ull * 1000 * 1000 * 1000;
 // --------------------------------------- the host loop's kernels, a step each
 
 __device__ __forceinline__ MsStep ms_step(const MsArgs &a, int j) {
-    return ms_step(a, a.ctl->level, j, a.ctl->tmask);
+    return ms_step(a, a.ctl->level, j, a.ctl->tmask, false);
 }
 
 // Adds what the warps found to the level's counters.
@@ -131,10 +131,12 @@ __global__ void k_ms_roots(MsArgs a, MsInit in) {
     }
 }
 
+// (four blocks an SM, three for the two-group pull: at five and four the loops
+// spill: R-MAT scale 19's first pull 198 against 227 us)
 constexpr int kMsBuBlock = 256;
 
 template <bool kBypass, bool kEarly, bool kFilt, bool kWide = false>
-__global__ void __launch_bounds__(kMsBuBlock, kWide ? 4 : 5) k_ms_bu(MsArgs a, int j) {
+__global__ void __launch_bounds__(kMsBuBlock, kWide ? 3 : 4) k_ms_bu(MsArgs a, int j) {
     const MsStep x = ms_step(a, j);
     MsCounts cnt;
     ms_pull<kBypass, kEarly, kFilt, kWide>(a, x, a.ctl->grab, INT32_MAX, &a.ctl->work[x.L % 3], cnt);
@@ -663,6 +665,9 @@ alb_status msbfs_impl(alb_graph *g, const int32_t *roots, int32_t nroots, const 
     cudaStream_t stream = g->stream;
     const int block = o.block;
     const unsigned wide = (unsigned)(g->num_sms * std::max(1, 2048 / block));
+    // the cooperative kernel; a traced run of it records its levels on the
+    // device, so that the trace times the benchmarked form itself
+    const bool coop = o.loop != ALB_LOOP_HOST && !prof;
     MsInit in;
     std::memset(&in, 0, sizeof(in));
     for (int i = 0; i < nroots; i++) in.roots[i] = roots[i];
@@ -677,11 +682,17 @@ alb_status msbfs_impl(alb_graph *g, const int32_t *roots, int32_t nroots, const 
     in.active0 = s.active0;
     in.push_budget = s.m_in / kPushDiv;
     {
-        // words per run of the pull: about three runs per warp, 1 .. 32
-        // (RMAT s22: 8 beats 32 by 7 %; s24: 32 beats 8 by 2 %, where longer runs
-        // save counter round trips and still leave every warp busy)
-        const int64_t warps = (int64_t)32 * g->num_sms;
-        in.grab = (int32_t)std::max<int64_t>(1, std::min<int64_t>(32, s.nwords / (3 * warps)));
+        // words per run of the pull: about three runs per resident warp, up to
+        // 32 (RMAT s22: 8 beats 32 by 7 %; s24: 32 beats 8 by 2 %, where longer
+        // runs save counter round trips and still leave every warp busy). The
+        // cooperative kernel, whose teams take the widest words first, goes
+        // down to 1; the host loop's kernels to 8: with fewer words a run a
+        // window's wide first word comes up late (s19: a level 205 -> 295 us).
+        const int per = resident_blocks((const void *)k_ms_bu<true, true, false>, kMsBuBlock);
+        const int64_t warps = coop ? (int64_t)32 * g->num_sms
+                                   : (int64_t)std::max(per, 1) * (kMsBuBlock / 32) * g->num_sms;
+        in.grab = (int32_t)std::max<int64_t>(coop ? 1 : kGrabWords,
+                                             std::min<int64_t>(32, s.nwords / (3 * warps)));
     }
     if (const char *e = std::getenv("ALB_MS_PUSH_DIV")) {  // tuning: 0 turns the push off
         const long long dv = std::atoll(e);
@@ -689,9 +700,6 @@ alb_status msbfs_impl(alb_graph *g, const int32_t *roots, int32_t nroots, const 
     }
     const int32_t level_cap = (int32_t)std::min<int64_t>(g->n + 1, INT32_MAX - 1);
     in.level_cap = level_cap;
-    // the cooperative kernel; a traced run of it records its levels on the
-    // device, so that the trace times the benchmarked form itself
-    const bool coop = o.loop != ALB_LOOP_HOST && !prof;
     const bool gtrace = trace && coop;
     in.gtrace = gtrace ? 1 : 0;
     in.unused = nroots >= 64 ? 0ull : ~((1ull << nroots) - 1);
