@@ -338,11 +338,11 @@ def run_ours(args, rank: int, world: int, dist) -> None:
 
 def roofline(dg, roots, d_ms, policy) -> dict:
     """Dominant kernel of the batched step: the bottom-up level of the 64-root
-    BFS (k_ms_bu over the slices, then the long-row head/tail passes and their
-    fold-in, the push of the pushed roots and the frontier sampling). Bytes
-    are counted by the kernels themselves (the model in include/albba.h); time
-    is CUDA events around the level's launches on the graph's stream, from the
-    host-driven trace run with the bench's policy."""
+    BFS (the pull over the slices, then the long-row head/tail passes and their
+    fold-in, the push of the pushed roots and the frontier sampling, all steps
+    of k_ms_grid). Bytes are counted by the kernel itself (the model in
+    include/albba.h); time is %globaltimer at the level's start and end, from a
+    traced run with the bench's policy."""
     import albba_gb300 as ab
     peak, kind = peaks()
     byts, us, nlev = 0, 0.0, 0
@@ -358,9 +358,8 @@ def roofline(dg, roots, d_ms, policy) -> dict:
                               "gbs": round(t.bytes / t.step_us / 1e3, 1)})
     gbs = byts / us / 1e3 if us > 0 else 0.0
     return {"bound": "hbm",
-            "kernel": "k_ms_bu + k_ms_bu_long + k_ms_bu_long_tail + k_ms_bu_long_fin "
-                      "+ k_ms_tq + k_ms_td<push> + k_ms_td_big<push> + k_ms_sample "
-                      "(64-root bottom-up level)",
+            "kernel": "k_ms_grid (64-root bottom-up level: pull, long rows, "
+                      "push of the pushed roots)",
             "achieved": gbs, "peak": peak, "unit": "GB/s", "frac": gbs / peak,
             "peak_kind": f"{kind} HBM copy bandwidth (burst)",
             "bytes_per_launch": byts / max(nlev, 1), "us_per_launch": us / max(nlev, 1),
@@ -433,8 +432,8 @@ def spmv_roofline(g, reps: int = 20) -> dict:
     t_floor, _ = median_us(rp1, g.col[lo:hi], val[lo:hi])
     byts = 12 * g.nnz + 24 * g.n
     gbs = byts / t / 1e3
-    return {"kernel": "k_spmv + k_spmv_long (fp64 SELL-32-sigma SpMV, y = A x)",
-            "bound": "the longest row's dependent fp64 fma chain (bit-exact order)",
+    return {"kernel": "k_spmv + k_spmv_long + k_spmv_hub (fp64 SELL-32-sigma SpMV, y = A x)",
+            "bound": "the longest row's in-order fp64 sum (bit-exact)",
             "achieved": gbs, "peak": peak, "unit": "GB/s", "frac": gbs / peak,
             "peak_kind": f"{kind} HBM copy bandwidth (burst)", "bytes_per_launch": byts,
             "us_per_launch": t, "stored_slots": stored, "entries": g.nnz,

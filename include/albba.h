@@ -152,8 +152,8 @@ alb_status alb_sell_long_export(const alb_graph *g, int64_t *nlong, int32_t *lro
 /* Level-loop driver. Single-root searches under either device-driven loop run
  * as one kernel for all levels (graphs of up to 2^16 vertices on one
  * thread-block cluster, larger ones on all SMs), except where a trace or the
- * pull without bypass is asked for: those, and the batched searches, run as
- * described here. */
+ * pull without bypass is asked for: those run as described here. Batched
+ * searches run as one kernel under both, traced or not. */
 #define ALB_LOOP_HOST 0       /* one set of launches per level, host decides */
 #define ALB_LOOP_GRAPH 1      /* CUDA graph with a device-driven while node */
 #define ALB_LOOP_PERSISTENT 2 /* one cooperative kernel for all levels */
@@ -251,10 +251,11 @@ alb_status alb_level_trace(const alb_graph *g, int32_t cap, alb_level_rec *out,
  * levels (host, n * 64 int32) is vertex-major: levels[v * 64 + i] = depth of
  * v from roots[i], -1 if unreached (and for i >= nroots); page-locked host
  * memory is written by the device directly, other host memory through a
- * device buffer and one copy. The level loop is a CUDA graph that decides
- * and launches every level on the device (ALB_LOOP_GRAPH, the default; the
- * host steps in only when the 32-level snapshot store fills) or host-driven
- * (ALB_LOOP_HOST: one small device-to-host read per level); the direction of
+ * device buffer and one copy. The search is one kernel that
+ * decides every level on the device (ALB_LOOP_GRAPH, the default, and
+ * ALB_LOOP_PERSISTENT; the host steps in only when the 32-level snapshot
+ * store fills) or host-driven (ALB_LOOP_HOST: one small device-to-host read
+ * per level); the direction of
  * each level is decided on the device (policy as for alb_bfs; the learned
  * policy uses selector 1). stats: reached = (vertex, root) pairs reached,
  * edges = sum over roots of push-side entries in the root's component. */
@@ -273,8 +274,8 @@ alb_status alb_msbfs64_device(alb_graph *g, const int32_t *roots, int32_t nroots
  * long rows) and Beamer thresholds. Levels only (no parents). A graph added
  * to a work list must outlive the list's runs. A graph whose bitmaps exceed
  * one CTA's shared memory (3 bits per vertex: above about 540K vertices)
- * runs its items one by one on the single-root path (alb_bfs_device,
- * CUDA-graph loop, the entry's alpha and beta) into the same output. */
+ * runs its items one by one on the single-root path (alb_bfs_device, the
+ * entry's alpha and beta) into the same output. */
 typedef struct alb_worklist alb_worklist;
 alb_status alb_worklist_create(alb_worklist **out);
 void alb_worklist_destroy(alb_worklist *w);
