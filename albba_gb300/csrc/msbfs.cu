@@ -665,9 +665,11 @@ alb_status msbfs_impl(alb_graph *g, const int32_t *roots, int32_t nroots, const 
     cudaStream_t stream = g->stream;
     const int block = o.block;
     const unsigned wide = (unsigned)(g->num_sms * std::max(1, 2048 / block));
-    // the cooperative kernel; a traced run of it records its levels on the
-    // device, so that the trace times the benchmarked form itself
-    const bool coop = o.loop != ALB_LOOP_HOST && !prof;
+    // the cooperative kernel; a run of it traced under ALB_LOOP_GRAPH records
+    // its levels on the device, so that the trace times the benchmarked form
+    // itself (one under ALB_LOOP_PERSISTENT has the active words too, which only
+    // the host-driven loop records)
+    const bool coop = o.loop != ALB_LOOP_HOST && !prof && !(trace && o.loop == ALB_LOOP_PERSISTENT);
     MsInit in;
     std::memset(&in, 0, sizeof(in));
     for (int i = 0; i < nroots; i++) in.roots[i] = roots[i];

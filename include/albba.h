@@ -153,7 +153,8 @@ alb_status alb_sell_long_export(const alb_graph *g, int64_t *nlong, int32_t *lro
  * as one kernel for all levels (graphs of up to 2^16 vertices on one
  * thread-block cluster, larger ones on all SMs), except where a trace or the
  * pull without bypass is asked for: those run as described here. Batched
- * searches run as one kernel under both, traced or not. */
+ * searches run as one kernel under both (traced ones under ALB_LOOP_GRAPH; a
+ * trace under ALB_LOOP_PERSISTENT is host-driven). */
 #define ALB_LOOP_HOST 0       /* one set of launches per level, host decides */
 #define ALB_LOOP_GRAPH 1      /* CUDA graph with a device-driven while node */
 #define ALB_LOOP_PERSISTENT 2 /* one cooperative kernel for all levels */
