@@ -282,6 +282,7 @@ constexpr int kTile = 256, kPer = kTile / 32;  // lane l: entries 8l .. 8l + 7
 constexpr int kHubFeed = 3, kHubScan = 3;      // warps that load, that scan
 constexpr int kHubThreads = 32 * (1 + kHubFeed + kHubScan);
 constexpr int kRunSeq = 8;
+constexpr int kNoGuess = -2;  // near no exponent
 
 struct HubTile {
     double v[kPer][32], x[kPer][32];
@@ -388,16 +389,18 @@ __global__ void __launch_bounds__(kHubThreads)
         feed.start(beg + (wib - 1) * kTile + kPer * lane);
         if (wib <= 2) feed.hand(s_t[wib - 1]);
     }
-    if (threadIdx.x == 0) s_E[0] = s_E[1] = s_guess[0] = s_guess[1] = -2;  // near no exponent
+    if (threadIdx.x == 0) s_E[0] = s_E[1] = s_guess[0] = s_guess[1] = kNoGuess;
     double acc = 0.0;
     for (int64_t t = 0; t < ntile; t++) {
         __syncthreads();  // tiles t and t + 1 and tile t's scans are in place
         if (wib > kHubFeed) {
             const int E = s_E[(t + 1) & 1];  // of the sum after tile t - 1
-            if (t + 1 < ntile && E > 0)
+            // (a zero or subnormal sum has no scans, not even of exponent 1)
+            const bool scans = t + 1 < ntile && E > 0;
+            if (scans)
                 hub_scan(s_t[(t + 1) % 3], E + wib - kHubFeed - 2,
                          s_h[((t + 1) & 1) * kHubScan + wib - kHubFeed - 1]);
-            if (wib == kHubFeed + 1 && lane == 0) s_guess[(t + 1) & 1] = E;
+            if (wib == kHubFeed + 1 && lane == 0) s_guess[(t + 1) & 1] = scans ? E : kNoGuess;
             continue;
         }
         if (wib > 0) {
