@@ -20,7 +20,9 @@
 // 2^52 < A <= 2^53. Above 2^52 the exact sum lies at or above 2^52 - with A
 // exactly 2^52 it may lie below, where the grid is finer - and a sum within
 // u / 2 of 2^53 rounds to 2^53 on either side's grid; from there a step down
-// is on this grid again, and one up leaves the interval.
+// is on this grid again, and one up leaves the interval. In the last binade
+// 2^53 u is infinity, from which no step leads back: sums in it, like zero and
+// subnormal ones, are not run this way (chain_runs).
 #pragma once
 
 #include <cstdint>
@@ -28,6 +30,9 @@
 namespace alb {
 
 constexpr int64_t kChainOne = 1ll << 52;
+
+// Whether a sum of biased exponent E may be run on integers.
+__host__ __device__ inline bool chain_runs(int E) { return E > 0 && E < 0x7FE; }
 
 // High half of a 64 x 64-bit product.
 __host__ __device__ inline uint64_t chain_mulhi(uint64_t a, uint64_t b) {
@@ -59,9 +64,10 @@ __host__ __device__ inline ChainTerm chain_term(uint64_t v, uint64_t x) {
     return t;
 }
 
-// k = round(p / u) for acc of biased exponent E (1 .. 2046). stop: p / u
-// may reach 2^53 (256 of them still add up in 64 bits), or p is halfway between two multiples of u. No branch: the
-// shift held at 63 sends every |p| below u / 2 to 0.
+// k = round(p / u) for acc of biased exponent E (1 .. 2046). stop: p / u may
+// reach 2^53 (256 of them still add up in 64 bits), or p is halfway between two
+// multiples of u. No branch: the shift held at 63 sends every |p| below u / 2
+// to 0.
 __host__ __device__ inline int64_t chain_round(int64_t h, int32_t e, int E, bool &stop) {
     int d = E + 1031 - e;
     stop = d < 9;

@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(kHubThreads)
             const bool ready = (unsigned)(E - guess + 1) < 3u;
             // (a scan for an exponent that was not prepared pays only where
             // the sum stands clear of its terms)
-            if (E > 0 && E < 0x7FF && (ready || E == E0 || E == E1 || E >= ep + 4)) {
+            if (chain_runs(E) && (ready || E == E0 || E == E1 || E >= ep + 4)) {
                 int h = ahead + E;
                 if (!ready) {
                     if (E != E0 && E != E1) {

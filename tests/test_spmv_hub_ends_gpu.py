@@ -1,7 +1,7 @@
 """The ends of the binades in which the CTA-per-row SpMV adds integers: sums
-that leave the subnormals slowly, and that stay zero for whole tiles before the
-smallest normal terms come. y equals the oracle's in-order chain bit for bit
-(tolerance zero)."""
+that leave the subnormals slowly, that stay zero for whole tiles before the
+smallest normal terms come, and that round to infinity and meet terms of the
+other sign. y equals the oracle's in-order chain bit for bit (tolerance zero)."""
 from __future__ import annotations
 
 import numpy as np
@@ -13,6 +13,7 @@ import oracle
 pytestmark = pytest.mark.gpu
 
 N = 5000  # one row: longer than any bound below which a row is summed by a lane
+MAX = np.finfo(np.float64).max
 
 
 def _spmv(rows):
@@ -60,3 +61,21 @@ def test_zeros_for_tiles_then_the_smallest_normals(exp, sign):
         x[first + 3:first + 500] = 2.0**-1060  # stays in the lowest binades for a while
         rows.append((v, x))
     _spmv(rows)
+
+
+@pytest.mark.parametrize("sign", [1.0, -1.0])
+@pytest.mark.parametrize("at", [20, 250, 256, 300, 700, 2000])
+def test_a_sum_that_rounds_to_infinity_stays_there(at, sign):
+    """The largest finite number, zeros, one last place up (infinity), and terms
+    of the other sign, which an infinite sum no longer feels."""
+    rows = []
+    for up, down, gap in ((2.0**971, 2.0**975, 1), (2.0**971, 2.0**975, 40), (2.0**971, 2.0**1000, 1),
+                          (1.5 * 2.0**970, 2.0**971, 1), (2.0**970, 2.0**971, 1), (2.0**969, 2.0**971, 1)):
+        v = np.zeros(N)
+        v[0] = MAX
+        v[at] = up
+        v[at + gap] = -down
+        v[at + gap + 200] = -2.0**1000
+        rows.append((sign * v, np.ones(N)))
+    want = _spmv(rows)
+    assert np.all(np.isinf(want[:5])) and np.isfinite(want[5])
