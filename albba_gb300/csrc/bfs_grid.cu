@@ -108,6 +108,11 @@ __device__ __forceinline__ List list_at(Pool &pool, int par) {
 
 // ------------------------------------------------------------- the barriers
 
+// The counting barriers that one level can have, each with four sums of its
+// own in the level's row of GridSlots::acc: a block may add to the next one's
+// while another still reads back the last one's.
+enum Sums : int { kSumLevel = 0, kSumLong = 4, kSumFits = 8, kSumActive = 12 };
+
 constexpr unsigned long long kBarFailed = 1ull << 62;  // a wait gave up
 // The arrival counter's word of a.bar, a line apart from the one that the
 // traced persistent kernel counts on (and starts from 0 each time).
@@ -1182,7 +1187,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bfs_grid(BfsArgs a, InitParams 
             if (!all) {  // does every block's share fit?
                 const bool no = (k & kEdgeMask) > (unsigned)cap || (k >> kRowShift) > (unsigned)kListRows;
                 put_counts(s, threadIdx.x == 0 && no, 0, 0, 0);
-                if (!(ok = barrier(a, s, L, acc + 8))) break;
+                if (!(ok = barrier(a, s, L, acc + kSumFits))) break;
                 lists = s.n == 0;
             }
             // both bitmaps are empty while lists are used
@@ -1232,7 +1237,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bfs_grid(BfsArgs a, InitParams 
                 leave_list(a, s, list_at(pool, par), s.nq[par], F, dir == ALB_DIR_TOPDOWN ? Q : nullptr,
                            &a.ctl->qn[L % 3], big);
                 count_active(a, s);
-                if (!(ok = barrier(a, s, L, acc + 4, big))) break;
+                if (!(ok = barrier(a, s, L, acc + kSumActive, big))) break;
                 if (threadIdx.x == 0) s.c.active_words = (int64_t)s.n;
             }
             if (dir == ALB_DIR_TOPDOWN) {
@@ -1258,7 +1263,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bfs_grid(BfsArgs a, InitParams 
             } else {
                 if (long_left) {
                     pull_long(a, s, F, big);
-                    if (!(ok = barrier(a, s, L, acc + 4, big))) break;
+                    if (!(ok = barrier(a, s, L, acc + kSumLong, big))) break;
                     long_left = (int64_t)s.n;
                     if (s.nbig) {
                         pull_long_tail(a, F, s.nbig);
@@ -1276,7 +1281,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bfs_grid(BfsArgs a, InitParams 
                 next_form = kMap;
             }
         }
-        if (!(ok = barrier(a, s, L, acc))) break;
+        if (!(ok = barrier(a, s, L, acc + kSumLevel))) break;
         if (ctl) end_level(next_form);
         __syncthreads();
         if (s.c.done) break;
