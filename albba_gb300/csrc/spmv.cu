@@ -34,6 +34,7 @@
 #include <cmath>
 #include <cstring>
 #include <functional>
+#include <utility>
 #include <vector>
 
 #include "chain.cuh"
@@ -57,7 +58,7 @@ struct alb_sellmat {
     double *val = nullptr;         // values, same layout
     double *dx = nullptr, *dy = nullptr;  // staging for host vectors
     int64_t nlong = 0;             // rows longer than kSpLong
-    int64_t nhub = 0;              // the first of them, CTA per row (hub_threshold)
+    int64_t nhub = 0;              // the first of them, CTA per row (hub_rows)
     int32_t *lrow = nullptr;       // their row ids, longest first
     int64_t *lptr = nullptr;       // first entries in lcol / lval: of each hub (a multiple of
                                    // 8), then of each slice of 32 other long rows (of 128)
@@ -204,17 +205,20 @@ __global__ void __launch_bounds__(kSpBlock)
 }
 
 // Lane per long row, 32 rows of similar length per warp (longest first),
-// interleaved as in a slice. Bound: the longest row's chain, about 58 ns per
+// interleaved as in a slice. Bound: the longest row's chain, 52 to 75 ns per
 // entry. Every load has to land within the chain time of the groups before
 // it: columns are requested 2 kLd groups of four entries ahead, values and x
-// gathers kLd groups (kLd x 4 fmas, near 2 us) ahead, all in registers. Rings
-// in shared memory (cp.async) left the SM's L1 too small to hold the gathers
-// in flight: 1.5 ms at R-MAT scale 22 instead of 0.7, and 6 ms with the
-// slices' gathers beside it.
+// gathers kLd groups (kLd x 4 fmas) ahead, all in registers. Eight groups (2
+// us) where the matrix has no hub rows; four beside hubs, whose CTAs (and the
+// slices') then find more registers free. At 4 / 8: 900 rows of 4,000 entries
+// 271 / 241 us, 3,000 of 30,000 2,314 / 1,974; R-MAT scale 22, which has hubs,
+// 1,910 / 1,961. Rings in shared memory (cp.async) left the SM's L1 too small
+// to hold the gathers in flight: 1.5 ms at R-MAT scale 22 instead of 0.7, and 6
+// ms with the slices' gathers beside it.
 constexpr int kSpLongBlock = 32;  // one warp per CTA
 constexpr int kLb = 8;            // hub rows are padded to this many entries
-constexpr int kLd = 4;
 
+template <int kLd>
 __global__ void __launch_bounds__(kSpLongBlock)
     k_spmv_long(int64_t nrows, const int32_t *lrow, const int64_t *moff, const int32_t *llen,
                 const int32_t *lcol, const double *lval, const double *x, double *y) {
@@ -276,8 +280,10 @@ __global__ void __launch_bounds__(kSpLongBlock)
 // does so about 8 sqrt(N) times) one fma and another look; the sum mostly
 // moves between neighbouring binades, so the scans for them are at hand, and
 // warp 0 scans for any other exponent itself (the last two are kept). After a
-// step that leaves the sum small against its term, kRunSeq entries are done
-// by fma: there every second entry would end a run.
+// step that leaves the sum small against its term, or a run of fewer than
+// kRunSeq entries, kRunSeq are done by fma: a look costs as much as six, and
+// there the next would find little (150 rows of 1,000 signed terms 87 -> 78 us,
+// R-MAT scale 22 2,307 -> 2,205).
 constexpr int kTile = 256, kPer = kTile / 32;  // lane l: entries 8l .. 8l + 7
 constexpr int kHubFeed = 3, kHubScan = 3;      // warps that load, that scan
 constexpr int kHubThreads = 32 * (1 + kHubFeed + kHubScan);
@@ -420,7 +426,7 @@ __global__ void __launch_bounds__(kHubThreads)
         while (s < cnt) {
             const uint64_t ab = (uint64_t)__double_as_longlong(acc);
             const int E = (int)(ab >> 52) & 0x7FF;
-            int run = kRunSeq;
+            int run = kRunSeq, got = 0;  // got: entries that the look found
             const bool ready = (unsigned)(E - guess + 1) < 3u;
             // (a scan for an exponent that was not prepared pays only where
             // the sum stands clear of its terms)
@@ -456,6 +462,7 @@ __global__ void __launch_bounds__(kHubThreads)
                 // the first entry that ends the run (cnt: none)
                 const int f = (int)__reduce_min_sync(
                     kFull, out ? (unsigned)(kPer * lane + __ffs(out) - 1) : (unsigned)cnt);
+                got = f - s;
                 if (f > s) {  // entries s .. f - 1 (A == 2^53 carries into the exponent)
                     const int64_t w = (H.P[(f - 1) & 7][(f - 1) >> 3] ^ sg) + base + 1;
                     acc = __longlong_as_double(
@@ -465,13 +472,14 @@ __global__ void __launch_bounds__(kHubThreads)
                 if (s >= cnt) break;
                 run = 1;
             }
-            // the entry that ended the run; kRunSeq in all where the sum is
-            // left small against its term (exponents compared as integers: the
-            // fp64 pipe is the chain's)
+            // the entry that ended the run; kRunSeq in all after a short one or
+            // where the sum is left small against its term (exponents compared
+            // as integers: the fp64 pipe is the chain's)
             ep = T.e[s & 7][s >> 3] - 1023;
             acc = fma(T.v[s & 7][s >> 3], T.x[s & 7][s >> 3], acc);
             s++;
-            if (run == 1 && ((__double2hiint(acc) >> 20) & 0x7FF) >= ep + 2) continue;
+            if (run == 1 && got >= kRunSeq && ((__double2hiint(acc) >> 20) & 0x7FF) >= ep + 2)
+                continue;
             const int e = min(cnt, s + kRunSeq - 1);
             double pv[kRunSeq - 1], px[kRunSeq - 1];
 #pragma unroll
@@ -534,16 +542,50 @@ __global__ void k_sp_hub_fill(int64_t nlong, const int32_t *lrow, const int64_t 
     }
 }
 
-// Rows longer than this have a CTA each. Lane per row does 32 rows at once
-// but takes about 70 ns per entry of its longest; a hub takes 3 ns per entry
-// and, for signed terms, about 0.35 us at each of its some 10 sqrt(N) entries
-// that leave the binade, whatever the other rows are. So the line is drawn
-// where the longest lane-per-row chain ends well before the longest hub's, and
-// not lower: R-MAT scale 22 (longest row 163,186) takes 2.12 ms at 25 sqrt(N)
-// and at 12, 4.16 at 6, where 9,109 rows are hubs and their CTAs run in
-// waves; with positive terms 0.94, 0.84 and 1.25 ms.
-int32_t hub_threshold(int32_t longest) {
-    return std::max<int32_t>(kSpLong, (int32_t)(12.0 * std::sqrt((double)longest)));
+// How many of the long rows (len: their lengths, longest first) have a CTA
+// each. Lane per row does 32 rows at once but takes kLaneNs per entry of its
+// longest. A hub row's CTA takes 3 ns per entry and, for signed terms, 0.35 us
+// at each of the entries that leave the binade: about kHubNs per entry, and no
+// more than kHubRootNs times the root of the length, all in all. Up to two CTAs
+// an SM run as fast as one; more share the SM, and each then takes kShareNs per
+// entry and kShareRootNs per root of the time of all SMs together. Signed terms
+// are what is reckoned with: x is not known yet.
+//
+// The line between the two is drawn low, where the longest lane-per-row chain
+// ends well before the longest hub's, unless more rows than two an SM are above
+// it; then at the lowest length whose reckoned time is within a tenth of the
+// best. us, signed / positive terms: 100,000 rows of 1,000 entries take 418 lane
+// per row and 15,199 / 3,926 as hubs, 900 of 4,000 241 and 517 / 80, 600 of 30,000
+// 1,950 and 1,516 / 300, 150 of 1,000 59 and 81 / 20; R-MAT scale 22 (longest row
+// 163,186) 2.29 / 0.85 ms with the line at 12 sqrt(N), 2.22 / 0.81 at 25 and 4.10 /
+// 1.25 at 6, scale 16 (10,000) 0.34 / 0.07, 0.34 / 0.12 and 0.34 / 0.06.
+constexpr double kLaneNs = 58, kHubNs = 80, kHubRootNs = 4400, kShareNs = 0.032, kShareRootNs = 4.8;
+
+int64_t hub_rows(const std::vector<int32_t> &len, int num_sms) {
+    auto above = [&](double t) -> int64_t {  // rows longer than t
+        return std::lower_bound(len.begin(), len.end(), (int32_t)t, std::greater<int32_t>()) -
+               len.begin();
+    };
+    const double longest = len[0], low = std::max((double)kSpLong, 12.0 * std::sqrt(longest));
+    if (above(low) <= 2 * (int64_t)num_sms) return above(low);
+    auto alone = [](double n) { return std::min(kHubNs * n, kHubRootNs * std::sqrt(n)); };
+    std::vector<double> all(1, 0.0);  // all[k]: what the first k rows take of all SMs
+    for (int64_t i = 0; i < above(low); i++)
+        all.push_back(all.back() + kShareNs * len[i] + kShareRootNs * std::sqrt((double)len[i]));
+    std::vector<std::pair<int64_t, double>> line;  // rows above it, time
+    for (double t = low;; t *= 1.25) {
+        const int64_t k = above(t);
+        double ns = k < (int64_t)len.size() ? kLaneNs * len[(size_t)k] : 0.0;
+        if (k > 0) ns = std::max(ns, alone(longest));
+        if (k > 2 * (int64_t)num_sms) ns = std::max(ns, all[(size_t)k] + alone(len[(size_t)k - 1]) / 2);
+        line.emplace_back(k, ns);
+        if (k == 0) break;
+    }
+    double best = line[0].second;
+    for (const auto &l : line) best = std::min(best, l.second);
+    for (const auto &l : line)
+        if (l.second <= 1.1 * best) return l.first;
+    return 0;
 }
 
 alb_status build(alb_sellmat *m, const int64_t *rowptr, const int32_t *col, const double *val) {
@@ -642,9 +684,7 @@ alb_status build(alb_sellmat *m, const int64_t *rowptr, const int32_t *col, cons
                 srow[(size_t)i] = hrow[(size_t)order[(size_t)i]];
                 slen[(size_t)i] = (int32_t)hlen[(size_t)order[(size_t)i]];
             }
-            m->nhub = std::lower_bound(slen.begin(), slen.end(), hub_threshold(slen[0]),
-                                       std::greater<int32_t>()) -
-                      slen.begin();
+            m->nhub = hub_rows(slen, m->num_sms);
             // hubs: rows one after the other, each padded to kLb entries; the
             // others: slices of 32 rows, as wide as the first (longest) one
             for (int64_t i = 0; i < m->nhub; i++)
@@ -737,7 +777,8 @@ alb_status launch(alb_sellmat *m, const double *d_x, double *d_y, float *us) {
     }
     if (rest) {
         ALB_CK(cudaStreamWaitEvent(m->side2, m->fork, 0));
-        k_spmv_long<<<blocks_for(m->nlong - m->nhub, kSpC), kSpLongBlock, 0, m->side2>>>(
+        const auto f = hubs ? k_spmv_long<4> : k_spmv_long<8>;
+        f<<<blocks_for(m->nlong - m->nhub, kSpC), kSpLongBlock, 0, m->side2>>>(
             m->nlong - m->nhub, m->lrow + m->nhub, m->lptr + m->nhub, m->llen + m->nhub, m->lcol,
             m->lval, d_x, d_y);
         ALB_CK(cudaGetLastError());
