@@ -1407,9 +1407,8 @@ struct alb::CachedLoop {
 
 namespace alb {
 
-alb_status bfs_scratch_alloc(alb_graph *g) {
+static alb_status scratch_alloc(alb_graph *g) {
     BfsScratch &b = g->bfs;
-    if (b.ready) return ALB_OK;
     const int64_t n = g->n, nw = g->sell.nwords;
     // the three bitmaps in one allocation (one L2 window covers them), each
     // padded to 16 bytes: k_bu_smem copies a frontier bitmap whole
@@ -1457,8 +1456,21 @@ alb_status bfs_scratch_alloc(alb_graph *g) {
     b.trace_cap = (int32_t)std::min<int64_t>(n + 2, 1 << 16);
     ALB_TRY(dmalloc((void **)&b.trace, sizeof(alb_level_rec) * b.trace_cap, "level trace"));
     ALB_CK(cudaMallocHost((void **)&b.h_ctl, sizeof(BfsCtl)));
+    // the barrier counter's zero is there once and for all: on a stream that
+    // is being captured the memset has not run, and this returns the error
+    ALB_CK(cudaStreamSynchronize(g->stream));
     b.ready = true;
     return ALB_OK;
+}
+
+alb_status bfs_scratch_alloc(alb_graph *g) {
+    if (g->bfs.ready) return ALB_OK;
+    const alb_status rc = scratch_alloc(g);
+    if (rc != ALB_OK) {
+        bfs_scratch_free(g);
+        cudaGetLastError();  // (nothing may be waited for under a capture)
+    }
+    return rc;
 }
 
 void bfs_scratch_free(alb_graph *g) {
@@ -1867,13 +1879,12 @@ alb_status bfs_impl(alb_graph *g, int32_t root, const alb_bfs_opts &o, int32_t *
     alb_status lrc = ALB_OK;
     if (coop) {
         g->bfs.h_ctl->done = g->bfs.h_ctl->err = 0;
-        if (!g->bfs.vrec_ready) {  // once, on the first call; without memory for them, without
-            g->bfs.vrec_ready = true;
-            if (s.max_deg <= kRecMaxDeg &&
-                dmalloc((void **)&g->bfs.vrec, sizeof(int4) * (size_t)g->n, "push-row records") ==
-                    ALB_OK)
-                lrc = row_recs_launch(g, a, g->bfs.vrec, stream);
-        }
+        // once, on the first call that ends well (else they may not have been
+        // written); without memory for them, without
+        if (!g->bfs.vrec_ready && s.max_deg <= kRecMaxDeg &&
+            (g->bfs.vrec ||
+             dmalloc((void **)&g->bfs.vrec, sizeof(int4) * (size_t)g->n, "push-row records") == ALB_OK))
+            lrc = row_recs_launch(g, a, g->bfs.vrec, stream);
         const GridArgs x{(GridSlots *)g->bfs.slots, g->bfs.vrec, s.max_deg, s.m_out,
                          g->symmetric ? 1 : 0,
                          g->bfs.h_ctl, 0};
@@ -1902,6 +1913,7 @@ alb_status bfs_impl(alb_graph *g, int32_t root, const alb_bfs_opts &o, int32_t *
     ALB_CK(cudaEventRecord(g->ev1, stream));
     if (coop) {
         const alb_status rc = finish_call(g, o, step_us, outputs ? 2 : 1, false, st);
+        if (rc == ALB_OK) g->bfs.vrec_ready = true;
         // (after an error the arrival counter is left between two barriers)
         if (rc != ALB_OK) ALB_CK(cudaMemsetAsync(g->bfs.bar, 0, 256, stream));
         return rc;
