@@ -1880,11 +1880,14 @@ alb_status bfs_impl(alb_graph *g, int32_t root, const alb_bfs_opts &o, int32_t *
     if (coop) {
         g->bfs.h_ctl->done = g->bfs.h_ctl->err = 0;
         // once, on the first call that ends well (else they may not have been
-        // written); without memory for them, without
-        if (!g->bfs.vrec_ready && s.max_deg <= kRecMaxDeg &&
-            (g->bfs.vrec ||
-             dmalloc((void **)&g->bfs.vrec, sizeof(int4) * (size_t)g->n, "push-row records") == ALB_OK))
-            lrc = row_recs_launch(g, a, g->bfs.vrec, stream);
+        // written); without memory for them, without, and without a message
+        if (!g->bfs.vrec_ready && s.max_deg <= kRecMaxDeg) {
+            const std::string said = alb_last_error();
+            if (!g->bfs.vrec && dmalloc((void **)&g->bfs.vrec, sizeof(int4) * (size_t)g->n,
+                                        "push-row records") != ALB_OK)
+                set_error("%s", said.c_str());
+            if (g->bfs.vrec) lrc = row_recs_launch(g, a, g->bfs.vrec, stream);
+        }
         const GridArgs x{(GridSlots *)g->bfs.slots, g->bfs.vrec, s.max_deg, s.m_out,
                          g->symmetric ? 1 : 0,
                          g->bfs.h_ctl, 0};
