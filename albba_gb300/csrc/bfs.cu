@@ -1890,6 +1890,7 @@ alb_status bfs_impl(alb_graph *g, int32_t root, const alb_bfs_opts &o, int32_t *
         }
         const GridArgs x{(GridSlots *)g->bfs.slots, g->bfs.vrec, s.max_deg, s.m_out,
                          g->symmetric ? 1 : 0,
+                         o.policy == ALB_POLICY_LEARNED && a.mlp && o.loop == ALB_LOOP_GRAPH ? 1 : 0,
                          g->bfs.h_ctl, 0};
         if (lrc == ALB_OK) lrc = grid_launch(g, a, ip, x, stream);
     } else if (o.loop == ALB_LOOP_HOST) {

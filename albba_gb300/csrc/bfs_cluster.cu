@@ -70,6 +70,7 @@ struct Shared {
     int level, dir, done, lists;  // lists: the level runs on lists, not on bitmaps
     unsigned nf, mf;
     Counts cnt[2];                // by level parity: what this CTA found
+    unsigned longest[2];          // and its longest row, at list levels
     unsigned next_word;
     unsigned nq[2];               // list counters (rows, edges) by level parity
     int even;                     // the lists are evened out before the level
@@ -369,10 +370,13 @@ __device__ void pull_words(const BfsArgs &a, Shared &s, cg::cluster_group &cl, i
 //
 // A small frontier (kListCap edges at most in any CTA, an edge per thread) is
 // kept as one list per CTA, in shared memory: the CTA that claims a vertex
-// pushes it at the next level, and lists that grew apart are evened out. A target is claimed by the compare-and-swap that moves its level
-// from -1, and its row's bounds and id are requested together with it, so a
-// level is two round trips to L2 and one barrier. The bitmaps go stale
-// and are rebuilt from the levels when a level needs them (lists_to_maps).
+// pushes it at the next level, and lists that grew apart are evened out. A
+// target is claimed by the compare-and-swap that moves its level from -1, and
+// its row's bounds and id are requested together with it, so a level is two
+// round trips to L2 and one barrier. The bitmaps go stale
+// and are rebuilt from the levels when a level needs them (lists_to_maps); under
+// the learned policy, to which the words with an unvisited row are a feature,
+// the visited words are kept up by the CTAs that own them.
 
 __device__ __forceinline__ void append(List &q, unsigned *nq, int32_t st, int32_t d, int32_t ou) {
     const unsigned at = atomicAdd(nq, (1u << kRowShift) | min((unsigned)d, kEdgeMask >> 10));
@@ -420,21 +424,28 @@ __device__ void even_lists(Shared &s, cg::cluster_group &cl, int rank, int nctas
     __syncthreads();
 }
 
-__device__ void list_level(const BfsArgs &a, Shared &s, int L) {
+// V: the visited words, per of them a CTA (kLearned).
+template <bool kLearned>
+__device__ void list_level(const BfsArgs &a, Shared &s, cg::cluster_group &cl, int L, uint32_t *V,
+                           int per) {
     const List &q = s.q[L & 1];
     const unsigned cnt = s.nq[L & 1];
     const int nq = (int)(cnt >> kRowShift), e = (int)threadIdx.x;
-    int32_t st = 0, len = 0, id = 0, in_len = 0;
+    int32_t v = -1, st = 0, len = 0, id = 0, in_len = 0;
+    uint32_t word = kFull;  // the target's visited word before
     bool claimed = false;
     if (e < (int)(cnt & kEdgeMask)) {
         int j = 0;  // the last row that starts at or before edge e (rows
                     // without edges share their start with the next one)
         for (int step = kListCap / 2; step > 0; step >>= 1)
             if (j + step < nq && q.off[j + step] <= e) j += step;
-        int32_t v = __ldg(a.pcol + q.st[j] + (e - q.off[j]));
+        v = __ldg(a.pcol + q.st[j] + (e - q.off[j]));
         ALB_CHECK_ID(v, a.n, -1, &a.ctl->err);
         if (v >= 0) {
             const int32_t old = atomicCAS(a.level_pos + v, -1, L + 1);
+            // (visited when the level ends, whoever claims it)
+            if (kLearned)
+                word = atomicOr(cl.map_shared_rank(V, (v >> 5) / per) + (v >> 5), 1u << (v & 31));
             const uint32_t cur = __ldcg(a.parent_pos + v), ou = (uint32_t)q.ou[j];
             st = (int32_t)__ldg(a.prow + v);
             len = (int32_t)__ldg(a.prow + v + 1) - st;
@@ -445,17 +456,21 @@ __device__ void list_level(const BfsArgs &a, Shared &s, int L) {
         }
     }
     if (claimed) append(s.q[(L + 1) & 1], &s.nq[(L + 1) & 1], st, len, id);
+    Counts &k = s.cnt[L & 1];
+    if (kLearned) {
+        const unsigned full = __ballot_sync(kFull, word != kFull && (word | (1u << (v & 31))) == kFull);
+        if (lane_id() == 0 && full) atomicAdd(&k.full, __popc(full));
+    }
     if (!__any_sync(kFull, claimed)) return;
     const unsigned n = __popc(__ballot_sync(kFull, claimed));
     const unsigned mo = __reduce_add_sync(kFull, claimed ? (unsigned)len : 0u);
     const unsigned mi = __reduce_add_sync(kFull, claimed ? (unsigned)in_len : 0u);
     const unsigned longest = __reduce_max_sync(kFull, claimed ? (unsigned)len : 0u);
     if (lane_id() == 0) {
-        Counts &k = s.cnt[L & 1];
         atomicAdd(&k.n, n);
         atomicAdd(&k.mo, mo);
         atomicAdd(&k.mi, mi);
-        atomicMax(&k.full, longest);  // (no words are counted at a list level)
+        atomicMax(&s.longest[L & 1], longest);
     }
 }
 
@@ -488,8 +503,9 @@ struct State {
 // The next level's direction and form (warp 0). most: the largest number of
 // edges any one CTA's list holds (after a bitmap level, the frontier's edges
 // or rows: any CTA might get them all).
+template <bool kLearned>
 __device__ void next_level(Shared &s, const State &t, const BfsArgs &a, const InitParams &in,
-                           bool learned, unsigned most) {
+                           unsigned most) {
     BfsCtl c;
     c.level = t.level;
     c.prev_dir = t.prev_dir;
@@ -507,7 +523,7 @@ __device__ void next_level(Shared &s, const State &t, const BfsArgs &a, const In
     c.feat_mean_deg = in.mean_deg;
     c.feat_skew = in.skew;
     int dir;
-    if (learned && s.mlp.loaded()) {
+    if (kLearned && s.mlp.loaded()) {
         float f[kMlpIn];
         level_features_warp(c, f);
         dir = s.mlp.select(f);
@@ -525,6 +541,8 @@ __device__ void next_level(Shared &s, const State &t, const BfsArgs &a, const In
     }
 }
 
+// kLearned: the learned policy, and weights may be loaded.
+template <bool kLearned>
 __global__ void __launch_bounds__(kThreads, 1)
     k_bfs_cluster(BfsArgs a, InitParams in, int32_t *out_level, int32_t *out_parent,
                   BfsCtl *result) {
@@ -549,9 +567,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         a.level_pos[p] = -1;
         a.parent_pos[p] = kFull;
     }
-    const bool learned = in.policy == ALB_POLICY_LEARNED && a.mlp;
-    if (learned) s.mlp.load(a.mlp);
+    if (kLearned) s.mlp.load(a.mlp);
     if (threadIdx.x < 8) reinterpret_cast<unsigned *>(s.cnt)[threadIdx.x] = 0;
+    if (threadIdx.x < 2) s.longest[threadIdx.x] = 0;
     __syncthreads();
     State t;
     const uint32_t rbit = 1u << (rp & 31), rold = V[rp >> 5];
@@ -574,7 +592,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (rank == 0) a.ctl->err = 0;
         s.done = 0;
     }
-    if (threadIdx.x < 32) next_level(s, t, a, in, learned, t.mf);
+    if (threadIdx.x < 32) next_level<kLearned>(s, t, a, in, t.mf);
     cl.sync();
     bool listed = false;  // the lists hold the frontier, the bitmaps are stale
     while (true) {
@@ -596,10 +614,13 @@ __global__ void __launch_bounds__(kThreads, 1)
             listed = false;
         }
         if (lists) {
-            if (!listed) maps_to_lists(a, s, F, L & 1, w0, w1);
-            else if (s.even) even_lists(s, cl, rank, nctas, L & 1);
+            if (!listed) {
+                maps_to_lists(a, s, F, L & 1, w0, w1);
+                // (the last level's visited bits are in before others claim)
+                if (kLearned) cl.sync();
+            } else if (s.even) even_lists(s, cl, rank, nctas, L & 1);
             listed = true;
-            list_level(a, s, L);
+            list_level<kLearned>(a, s, cl, L, V, per);
         } else if (dir == ALB_DIR_TOPDOWN) {
             for (int w = threadIdx.x; w < nw; w += kThreads) N[w] = 0;
             push_level(a, s, F, V, N, w0, w1, rank, nctas, s.nf <= kSplitRows);
@@ -615,7 +636,10 @@ __global__ void __launch_bounds__(kThreads, 1)
             if ((int)threadIdx.x < nctas) k = cl.map_shared_rank(&s, threadIdx.x)->cnt[L & 1];
             const unsigned most = lists ? __reduce_max_sync(kFull, k.mo) : 0;
             if (lists) {
-                const unsigned longest = __reduce_max_sync(kFull, k.full);
+                unsigned longest = 0;
+                if ((int)threadIdx.x < nctas)
+                    longest = cl.map_shared_rank(&s, threadIdx.x)->longest[L & 1];
+                longest = __reduce_max_sync(kFull, longest);
                 const unsigned upto = warp_inclusive_scan(k.n);
                 const unsigned tot = __shfl_sync(kFull, upto, 31);
                 if ((int)threadIdx.x < nctas) s.before[threadIdx.x] = upto - k.n;
@@ -624,7 +648,6 @@ __global__ void __launch_bounds__(kThreads, 1)
                     s.even = most > kListEven && nctas > 1 &&
                              (tot / nctas + 1) * (unsigned long long)longest <= kListCap;
                 }
-                k.full = 0;
             }
             t.prev_nf = t.nf;
             t.nf = __reduce_add_sync(kFull, k.n);
@@ -642,9 +665,10 @@ __global__ void __launch_bounds__(kThreads, 1)
                 // (the other parity's counts were read by everyone before the
                 // last barrier)
                 s.cnt[(L + 1) & 1] = Counts{0, 0, 0, 0};
+                s.longest[(L + 1) & 1] = 0;
                 s.done = t.nf == 0 || t.level >= in.level_cap;
             }
-            next_level(s, t, a, in, learned, lists ? most : max(t.mf, t.nf));
+            next_level<kLearned>(s, t, a, in, lists ? most : max(t.mf, t.nf));
         } else if (!lists) {
             for (int w = threadIdx.x - 32; w < nw; w += kThreads - 32) V[w] |= N[w];
         }
@@ -678,11 +702,13 @@ int cluster_ctas(int64_t nw) {
 // Dynamic shared memory: the CTA's state and the three bitmaps.
 size_t map_bytes(int64_t nw) { return sizeof(Shared) + sizeof(uint32_t) * 3 * (size_t)nw; }
 
-cudaError_t allow_cluster() {
-    cudaError_t e = cudaFuncSetAttribute(k_bfs_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
+using Kernel = void (*)(BfsArgs, InitParams, int32_t *, int32_t *, BfsCtl *);
+
+cudaError_t allow_cluster(Kernel f) {
+    cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)map_bytes(kClusterMaxN / 32));
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_bfs_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     return e;
 }
 
@@ -710,9 +736,12 @@ bool cluster_ready(int device) {
     if (it != known.end()) return it->second;
     cudaLaunchAttribute at;
     const cudaLaunchConfig_t cfg = config(kMaxCtas, map_bytes(kClusterMaxN / 32), nullptr, at);
-    int n = 0;
-    const bool ok = allow_cluster() == cudaSuccess &&
-                    cudaOccupancyMaxActiveClusters(&n, k_bfs_cluster, &cfg) == cudaSuccess && n >= 1;
+    bool ok = true;
+    for (Kernel f : {k_bfs_cluster<false>, k_bfs_cluster<true>}) {
+        int n = 0;
+        ok = ok && allow_cluster(f) == cudaSuccess &&
+             cudaOccupancyMaxActiveClusters(&n, f, &cfg) == cudaSuccess && n >= 1;
+    }
     if (!ok) cudaGetLastError();
     known[device] = ok;
     return ok;
@@ -722,17 +751,18 @@ bool cluster_ready(int device) {
 
 bool cluster_takes(const alb_graph *g, const alb_bfs_opts &o, const BfsArgs &a) {
     // (counters are 32 bits wide)
-    return g->n <= kClusterMaxN && g->sell.m_in <= INT32_MAX && g->sell.m_out <= INT32_MAX && o.loop != ALB_LOOP_HOST && !o.trace &&
-           o.policy != ALB_POLICY_BOTTOMUP_NOBYPASS && a.withhold_level < 0 && !a.short_bulk &&
+    return g->n <= kClusterMaxN && g->sell.m_in <= INT32_MAX && g->sell.m_out <= INT32_MAX &&
+           o.loop != ALB_LOOP_HOST && !o.trace && o.policy != ALB_POLICY_BOTTOMUP_NOBYPASS && a.withhold_level < 0 && !a.short_bulk &&
            cluster_ready(g->device);
 }
 
 alb_status cluster_launch(const BfsArgs &a, const InitParams &in, int32_t *d_level,
                           int32_t *d_parent, BfsCtl *result, cudaStream_t st) {
-    ALB_CK(allow_cluster());
+    const Kernel f = in.policy == ALB_POLICY_LEARNED && a.mlp ? k_bfs_cluster<true> : k_bfs_cluster<false>;
+    ALB_CK(allow_cluster(f));
     cudaLaunchAttribute at;
     const cudaLaunchConfig_t cfg = config(cluster_ctas(a.nwords), map_bytes(a.nwords), st, at);
-    ALB_CK(cudaLaunchKernelEx(&cfg, k_bfs_cluster, a, in, d_level, d_parent, result));
+    ALB_CK(cudaLaunchKernelEx(&cfg, f, a, in, d_level, d_parent, result));
     return ALB_OK;
 }
 

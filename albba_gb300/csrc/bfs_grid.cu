@@ -80,6 +80,7 @@ struct Shared {
     unsigned long long n, mo, mi, full, nbig;
     unsigned nq[2];
     unsigned cn, cmo, cmi, wide;  // a list level's claims in this block; rows too long for it
+    unsigned cwords;              // words of the visited bitmap that they filled (kExact)
     unsigned long long at;  // this block's place in a queue
     __align__(8) uint64_t bar;
     MlpCopy mlp;
@@ -207,10 +208,11 @@ static_assert(kMaxBlocks * kListCapMax < (1 << (kUneven - kVerts)) && kMaxBlocks
               "fields of the list word");
 
 // One warp, after the block's claims: arrives and waits, and leaves the sums in
-// s, exactly: acc holds the edges where the word does not. All lanes poll: with
+// s, exactly: acc holds the edges where the word does not, and filled words. All lanes poll: with
 // one lane waiting the warp came out of it in two parts, and every shuffle of
 // the decision that follows paid for bringing them together (12,900 cycles
 // instead of 2,000).
+template <bool kExact>
 __device__ __forceinline__ bool list_barrier(const BfsArgs &a, const GridArgs &x, Shared &s, int L,
                                              unsigned long long *word, unsigned long long *acc) {
     if (withheld(a, L)) return false;
@@ -224,7 +226,9 @@ __device__ __forceinline__ bool list_barrier(const BfsArgs &a, const GridArgs &x
     __syncwarp();
     if (lane == 0 && mo) atomicAdd(acc, (unsigned long long)mo);
     if (lane == 0 && !x.sym && mi) atomicAdd(acc + 1, (unsigned long long)mi);
+    if (kExact && lane == 0 && s.cwords) atomicAdd(acc + 2, (unsigned long long)s.cwords);
     if (lane == 0) s.cn = s.cmo = s.cmi = s.wide = 0;
+    if (kExact && lane == 0) s.cwords = 0;
     unsigned long long v = 0;
     if (lane == 0) v = atom_add_acq_rel(word, mine) + mine;
     v = __shfl_sync(kFull, v, 0);
@@ -243,13 +247,14 @@ __device__ __forceinline__ bool list_barrier(const BfsArgs &a, const GridArgs &x
     unsigned long long emo = v & ((1u << kVerts) - 1);
     if (any_over || any_uneven) emo = __ldcg(acc);
     const unsigned long long emi = x.sym ? emo : __ldcg(acc + 1);
+    const unsigned long long words = kExact ? __ldcg(acc + 2) : 0;
     if (lane == 0) {
         s.n = (v >> kVerts) & ((1u << (kUneven - kVerts)) - 1);
         s.uneven = any_uneven;
         s.over = any_over;
         s.mo = emo;
         s.mi = emi;
-        s.full = 0;
+        s.full = words;
     }
     __syncwarp();
     return ok;
@@ -411,18 +416,28 @@ __device__ __forceinline__ void claim(const BfsArgs &a, const Edges &E, int L, i
         was[k] = E.v[k] >= 0 ? atomicCAS(a.level_pos + E.v[k], -1, L + 1) : 0;
 }
 
+// kExact: the words of the visited bitmap that the claims fill are counted. How
+// many have an unvisited row is a feature of the learned policy, whose
+// directions under ALB_LOOP_GRAPH are those of the host-driven loop. Under
+// ALB_LOOP_PERSISTENT they are counted when the lists are left, as that loop
+// always did: the words that come back from the atomics, and the sum's way to
+// every block, are 10 % of the time of the grid of 2^24.
+template <bool kExact>
 __device__ __forceinline__ void list_level(const BfsArgs &a, const GridArgs &x, Shared &s,
                                            const Edges &E, const int32_t (&was)[kPer],
                                            const List &nx, unsigned *nnx, int L) {
     unsigned n = 0, mo = 0, mi = 0;
+    uint32_t vis[kPer];  // kExact: the claims' words before (full: no claim)
 #pragma unroll
     for (int k = 0; k < kPer; k++) {
+        vis[k] = kFull;
         if (E.v[k] < 0 || (was[k] != -1 && was[k] != L + 1)) continue;
         // (no look at the parent first: a list's frontier has few edges, and
         // each access to a large graph's arrays is a miss)
         atomicMin(a.parent_pos + E.v[k], E.ou[k]);
         if (was[k] != -1) continue;
-        atomicOr(a.vis + (E.v[k] >> 5), 1u << (E.v[k] & 31));
+        if (kExact) vis[k] = atomicOr(a.vis + (E.v[k] >> 5), 1u << (E.v[k] & 31));
+        else atomicOr(a.vis + (E.v[k] >> 5), 1u << (E.v[k] & 31));
         if (!append(nx, nnx, E.v[k], E.r[k].st, min(E.r[k].d, kListRow), E.r[k].id))
             overflow(a, E.v[k], L);
         if (E.r[k].d > kListRow) s.wide = 1;
@@ -434,15 +449,23 @@ __device__ __forceinline__ void list_level(const BfsArgs &a, const GridArgs &x, 
     n = __reduce_add_sync(kFull, n);
     mo = __reduce_add_sync(kFull, mo);
     if (!x.sym) mi = __reduce_add_sync(kFull, mi);
+    unsigned words = 0;
+    if (kExact) {
+#pragma unroll
+        for (int k = 0; k < kPer; k++)
+            words += vis[k] != kFull && (vis[k] | (1u << (E.v[k] & 31))) == kFull;
+        words = __reduce_add_sync(kFull, words);
+    }
     if (lane_id() == 0) {
+        if (kExact && words) atomicAdd(&s.cwords, words);
         atomicAdd(&s.cn, n);
         atomicAdd(&s.cmo, mo);
         if (mi) atomicAdd(&s.cmi, mi);
     }
 }
 
-// Bitmap words of this block that still have an unvisited row (the visited
-// bitmap's words are not watched while lists are used).
+// Bitmap words of this block that still have an unvisited row (while lists are
+// used they are not watched but under kExact).
 __device__ void count_active(const BfsArgs &a, Shared &s) {
     const int64_t w0 = a.nwords * blockIdx.x / gridDim.x, w1 = a.nwords * (blockIdx.x + 1) / gridDim.x;
     unsigned n = 0;
@@ -1087,6 +1110,7 @@ __device__ __forceinline__ void clear_next(const BfsArgs &a, const GridArgs &x, 
     }
 }
 
+template <bool kExact>
 __global__ void __launch_bounds__(kThreads, 1) k_bfs_grid(BfsArgs a, InitParams in, GridArgs x) {
     ALB_GRID_SHARED;
     __shared__ WarpRows wr[kWarps];
@@ -1123,7 +1147,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_bfs_grid(BfsArgs a, InitParams 
         s.level_cap = in.level_cap;
         s.learned = learned;
         s.cap = x.list_cap;
-        s.cn = s.cmo = s.cmi = s.wide = 0;
+        s.cn = s.cmo = s.cmi = s.wide = s.cwords = 0;
         mbar_init(&s.bar, 1);
         BfsCtl &c = s.c;
         c.prev_dir = c.dir = -1;
@@ -1211,13 +1235,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_bfs_grid(BfsArgs a, InitParams 
                     e += kListPass;
                     const bool more = e < (int)(cnt & kEdgeMask);
                     if (more) fetch_edges(a, x, cur, cap, cnt, e, E);
-                    list_level(a, x, s, now, was, nx, &s.nq[p ^ 1], l);
+                    list_level<kExact>(a, x, s, now, was, nx, &s.nq[p ^ 1], l);
                     if (!more) break;
                 }
                 __syncthreads();
                 if (ctl) {
-                    const bool k = list_barrier(a, x, s, l, x.slots->word[l % 3],
-                                                x.slots->acc[l % 3]);
+                    const bool k = list_barrier<kExact>(a, x, s, l, x.slots->word[l % 3],
+                                                        x.slots->acc[l % 3]);
                     if (lane_id() == 0) s.ok = k;
                     __syncwarp();
                     if (k) end_level(kList);
@@ -1369,13 +1393,14 @@ alb_status grid_launch(const alb_graph *g, const BfsArgs &a, const InitParams &i
     GridArgs x = args_in;
     x.list_cap = x.max_out <= kFewEdges ? kListCapMax : kListPass;
     const size_t smem = shared_bytes(a.nwords);
-    ALB_CK(cudaFuncSetAttribute(k_bfs_grid, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    void (*f)(BfsArgs, InitParams, GridArgs) = x.exact ? k_bfs_grid<true> : k_bfs_grid<false>;
+    ALB_CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)shared_bytes(kStageMax / 4)));
     BfsArgs aa = a;
     InitParams ii = in;
     GridArgs xx = x;
     void *args[] = {&aa, &ii, &xx};
-    ALB_CK(cudaLaunchCooperativeKernel((void *)k_bfs_grid, dim3((unsigned)g->num_sms),
+    ALB_CK(cudaLaunchCooperativeKernel((void *)f, dim3((unsigned)g->num_sms),
                                        dim3(kThreads), args, smem, st));
     return ALB_OK;
 }

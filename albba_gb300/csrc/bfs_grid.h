@@ -20,6 +20,7 @@ struct GridArgs {
     int64_t max_out;  // longest push row (0: not known)
     int64_t m_out;
     int32_t sym;      // push and pull rows are the same
+    int32_t exact;    // learned directions as the host-driven loop's (list_level)
     BfsCtl *result;   // page-locked: level, done, err, levels_*, reached, edges
     int32_t list_cap;  // set by grid_launch
 };

@@ -152,7 +152,10 @@ alb_status alb_sell_long_export(const alb_graph *g, int64_t *nlong, int32_t *lro
 /* Level-loop driver. Single-root searches under either device-driven loop run
  * as one kernel for all levels (graphs of up to 2^16 vertices on one
  * thread-block cluster, larger ones on all SMs), except where a trace or the
- * pull without bypass is asked for: those run as described here. Batched
+ * pull without bypass is asked for: those run as described here. The learned
+ * policy takes the host-driven loop's directions under ALB_LOOP_GRAPH; on all
+ * SMs under ALB_LOOP_PERSISTENT the words with an unvisited row, one of its
+ * features, are not counted while frontiers are small. Batched
  * searches run as one kernel under both (traced ones under ALB_LOOP_GRAPH; a
  * trace under ALB_LOOP_PERSISTENT is host-driven). */
 #define ALB_LOOP_HOST 0       /* one set of launches per level, host decides */
