@@ -74,7 +74,7 @@ struct Shared {
     // of the call: longest push row, rows and entries as GridArgs has them
     int64_t max_out, m_out;
     int level_cap, learned, cap;  // cap: edges of a list
-    int dir, form, lists, even, sparse, ok, over, uneven;
+    int dir, form, lists, even, sparse, scan, ok, over, uneven;
     Counts warp[kWarps];
     // sums of the last counting barrier; nbig: the big-row counter
     unsigned long long n, mo, mi, full, nbig;
@@ -775,16 +775,20 @@ __device__ void pull_long_tail(const BfsArgs &a, const uint32_t *F, unsigned lon
     }
 }
 
-// The group's first source in the frontier (-1: none).
-template <bool kStaged>
-__device__ __forceinline__ int32_t test_group(const uint32_t *F, const int4 &c) {
-    auto word = [&](int32_t v) { return kStaged ? F[v >> 5] : __ldcg(F + (v >> 5)); };
-    const uint32_t f0 = word(c.x), f1 = word(c.y), f2 = word(c.z), f3 = word(c.w);
+// The group's first source in the frontier (-1: none), f0 .. f3 its frontier words.
+__device__ __forceinline__ int32_t first_hit(const int4 &c, uint32_t f0, uint32_t f1, uint32_t f2,
+                                             uint32_t f3) {
     if ((f0 >> (c.x & 31)) & 1u) return c.x;
     if ((f1 >> (c.y & 31)) & 1u) return c.y;
     if ((f2 >> (c.z & 31)) & 1u) return c.z;
     if ((f3 >> (c.w & 31)) & 1u) return c.w;
     return -1;
+}
+template <bool kStaged>
+__device__ __forceinline__ int32_t test_group(const uint32_t *F, const int4 &c) {
+    auto word = [&](int32_t v) { return kStaged ? F[v >> 5] : __ldcg(F + (v >> 5)); };
+    const uint32_t f0 = word(c.x), f1 = word(c.y), f2 = word(c.z), f3 = word(c.w);
+    return first_hit(c, f0, f1, f2, f3);
 }
 
 // Word shape: a warp takes runs of words from the level's counter, lane l's
@@ -796,8 +800,13 @@ __device__ __forceinline__ int32_t test_group(const uint32_t *F, const int4 &c) 
 // 2^23 255 -> 243, scale 24 from a leaf 379 -> 367 and from a hub 614 -> 610;
 // equal runs of 8: 985, 248, 381, 643. Bound: the gathers of frontier bits, an
 // address per clock and SM (2^22 vertices of mean degree 8: 31 M in 108 us).
-template <bool kStaged>
-__device__ void pull_words(const BfsArgs &a, Shared &s, const uint32_t *F, uint32_t *N, int L,
+// kScan (pull_scan): rows are mostly read to their ends, and a wide slice's step
+// is a column load and two words' frontier tests one after the other; there both
+// words' frontier words are requested before either is tested, one round trip a
+// step instead of two. (Everywhere it costs registers that the kernel has not
+// got: a hub's search of R-MAT scale 22 146 -> 156 us.)
+template <bool kStaged, bool kScan>
+__device__ __forceinline__ void pull_words(const BfsArgs &a, Shared &s, const uint32_t *F, uint32_t *N, int L,
                            unsigned long long *ctr, bool sym) {
     constexpr int kW = 2;
     const int lane = lane_id();
@@ -878,13 +887,27 @@ __device__ void pull_words(const BfsArgs &a, Shared &s, const uint32_t *F, uint3
                     nx[t] = make_int4(p[t], p[t], p[t], p[t]);
                     if (act[t] && j + 1 < ng[t]) nx[t] = ld_stream(cp[t] + (int64_t)(j + 1) * C, pol);
                 }
+                uint32_t f[kW][4];
+                if (kScan) {
+#pragma unroll
+                    for (int t = 0; t < kW; t++) {
+                        if (!act[t]) continue;
+                        ALB_CHECK_ID4(c[t], a.nwords * 32, p[t], &a.ctl->err);
+                        f[t][0] = F[c[t].x >> 5], f[t][1] = F[c[t].y >> 5];
+                        f[t][2] = F[c[t].z >> 5], f[t][3] = F[c[t].w >> 5];
+                    }
+                }
 #pragma unroll
                 for (int t = 0; t < kW; t++) {
                     if (!act[t]) continue;
-                    ALB_CHECK_ID4(c[t], a.nwords * 32, p[t], &a.ctl->err);
                     // padding is the row itself, never in the frontier, and
                     // ends the row: the first hit is the smallest source
-                    found[t] = test_group<kStaged>(F, c[t]);
+                    if (kScan) {
+                        found[t] = first_hit(c[t], f[t][0], f[t][1], f[t][2], f[t][3]);
+                    } else {
+                        ALB_CHECK_ID4(c[t], a.nwords * 32, p[t], &a.ctl->err);
+                        found[t] = test_group<kStaged>(F, c[t]);
+                    }
                     act[t] = found[t] < 0 && c[t].w != p[t];
                     c[t] = nx[t];
                 }
@@ -916,6 +939,15 @@ __device__ void pull_words(const BfsArgs &a, Shared &s, const uint32_t *F, uint3
         }
     }
     put_counts(s, cn, mo, mi, full);
+}
+
+// The word shape for a frontier that few rows have a source in, as a function of
+// its own: the kernel around it keeps its registers.
+__device__ __noinline__ void pull_scan(BfsArgs a, const uint32_t *F, uint32_t *N, int L,
+                                       unsigned long long *ctr, bool sym) {
+    ALB_GRID_SHARED;
+    (void)pool;
+    pull_words<false, true>(a, s, F, N, L, ctr, sym);
 }
 
 // Row shape: the unvisited rows of 32 words, dealt out to the lanes.
@@ -1051,6 +1083,10 @@ __device__ __forceinline__ void next_level(Shared &s, const BfsCtl &c) {
         // (at 10 of 32 a uniform random graph of 2^24 takes 1,145 us, at 16 1,081;
         // at 24 one of 2^22 364 -> 420)
         s.sparse = c.nu < 16 * c.active_words;
+        // few rows have a source in the frontier: under a 32nd of the unvisited
+        // rows' entries point into it (bottom-up from a leaf of R-MAT of 2^22
+        // 1,344 -> 960 us, of 2^21 890 -> 620)
+        s.scan = 32 * c.mf < c.mu;
     }
 }
 
@@ -1115,7 +1151,10 @@ __device__ __forceinline__ void clear_next(const BfsArgs &a, const GridArgs &x, 
     }
 }
 
-template <bool kExact>
+// kScan: frontiers too large to stage may be pulled while they are small, as
+// under the bottom-up policy (pull_scan; the call alone, where it is never made,
+// costs the grid of 2^24 8 %).
+template <bool kExact, bool kScan>
 __global__ void __launch_bounds__(kThreads, 1) k_bfs_grid(BfsArgs a, InitParams in, GridArgs x) {
     ALB_GRID_SHARED;
     __shared__ WarpRows wr[kWarps];
@@ -1303,9 +1342,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_bfs_grid(BfsArgs a, InitParams 
                     pull_rows(a, s, pool.rows, F, N, L, x.sym);
                 } else if (a.nwords * 4 <= kStageMax) {
                     if (!(ok = stage_frontier(a, s, pool.stage, F, staged++ & 1))) break;
-                    pull_words<true>(a, s, pool.stage, N, L, work, x.sym);
+                    pull_words<true, false>(a, s, pool.stage, N, L, work, x.sym);
+                } else if (kScan && s.scan) {
+                    pull_scan(a, F, N, L, work, x.sym);
                 } else {
-                    pull_words<false>(a, s, F, N, L, work, x.sym);
+                    pull_words<false, false>(a, s, F, N, L, work, x.sym);
                 }
                 next_form = kMap;
             }
@@ -1398,7 +1439,10 @@ alb_status grid_launch(const alb_graph *g, const BfsArgs &a, const InitParams &i
     GridArgs x = args_in;
     x.list_cap = x.max_out <= kFewEdges ? kListCapMax : kListPass;
     const size_t smem = shared_bytes(a.nwords);
-    void (*f)(BfsArgs, InitParams, GridArgs) = x.exact ? k_bfs_grid<true> : k_bfs_grid<false>;
+    const bool scan = in.policy == ALB_POLICY_BOTTOMUP && a.nwords * 4 > kStageMax;
+    void (*f)(BfsArgs, InitParams, GridArgs) = x.exact ? k_bfs_grid<true, false>
+                                               : scan  ? k_bfs_grid<false, true>
+                                                       : k_bfs_grid<false, false>;
     ALB_CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)shared_bytes(kStageMax / 4)));
     BfsArgs aa = a;

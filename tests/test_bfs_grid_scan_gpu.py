@@ -1,5 +1,7 @@
-"""The cooperative kernel where it pushes many edges of a small graph: levels and
-parents against the oracle."""
+"""The cooperative kernel where it pulls for a frontier that few rows have a
+source in (bottom-up throughout, frontiers too large to stage in shared
+memory), and where it pushes many edges of a small graph, from hubs and
+leaves: levels and parents against the oracle."""
 from __future__ import annotations
 
 import numpy as np
@@ -23,6 +25,20 @@ def _check(g, dg, root, policy):
     lv, pa, st = dg.bfs(int(root), ab.bfs_opts(policy))
     olv, opa, nl = oracle.bfs(g.rowptr, g.col, int(root))
     assert np.array_equal(lv, olv) and np.array_equal(pa, opa) and st.num_levels == nl
+
+
+# (bitmaps are staged up to 1,572,864 vertices)
+@pytest.mark.parametrize("C_,sigma,long_row", [(32, 1024, 1024), (8, 64, 40), (64, 4096, 0)])
+@pytest.mark.parametrize("kind", ["rmat", "er", "edge"])
+def test_bottom_up_throughout(kind, C_, sigma, long_row):
+    g = {"rmat": lambda: ab.gen_rmat(21, 4, seed=5), "er": lambda: ab.gen_er(1_700_003, 6.0, seed=5),
+         "edge": lambda: ab.gen_er(1_572_865, 3.0, seed=6)}[kind]()
+    deg = np.diff(g.rowptr)
+    leaf = int(np.flatnonzero(deg == 1)[7])
+    with ab.Graph(g) as dg:
+        dg.sell_build(C_, sigma, long_row)
+        for root in (leaf, int(deg.argmax())):
+            _check(g, dg, root, "bottomup")
 
 
 @pytest.mark.parametrize("n,m", [(2000, 400_000), (33, 400), (20_001, 3_000_000), (70_001, 4_000_000)])
