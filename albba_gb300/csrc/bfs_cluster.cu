@@ -750,6 +750,14 @@ bool cluster_ready(int device) {
 }  // namespace
 
 bool cluster_takes(const alb_graph *g, const alb_bfs_opts &o, const BfsArgs &a) {
+    // Policies that push (or may) go to all SMs where there are many edges a
+    // vertex: 16 SMs push 2 M edges of 4,000 vertices in 189 us, all of them in
+    // 89, 33 M of 65,000 in 948 and 201 (learned 214 / 92, 99 / 86); around 100 a
+    // vertex, R-MAT of 2^15, learned is 75 / 83 and top-down 153 / 109. The other
+    // policies pull there: 38 / 60 and 93 / 83.
+    if ((o.policy == ALB_POLICY_TOPDOWN || o.policy == ALB_POLICY_LEARNED) &&
+        g->sell.m_out > 100 * g->n)
+        return false;
     // (counters are 32 bits wide)
     return g->n <= kClusterMaxN && g->sell.m_in <= INT32_MAX && g->sell.m_out <= INT32_MAX &&
            o.loop != ALB_LOOP_HOST && !o.trace && o.policy != ALB_POLICY_BOTTOMUP_NOBYPASS && a.withhold_level < 0 && !a.short_bulk &&
