@@ -17,9 +17,12 @@
 // time. 48 R-MAT graphs of 2^10 to 2^16 vertices, 8 roots each: 222 us; 3.5 ms
 // with 256 threads, a row per warp and a word per warp at a time.
 // Output: level arrays (original ids), one per item, concatenated in the
-// order items were added. Graphs whose bitmaps do not fit in one CTA's
-// shared memory are not refused: their items run one by one on the
-// device-driven single-root path (alb_bfs_device, the entry's alpha and beta) into the same output, before the launch.
+// order items were added. Graphs whose bitmaps do not fit in one CTA's shared
+// memory are not refused: their items run one by one on the device-driven
+// single-root path (alb_bfs_device, the entry's alpha and beta) into the same
+// output, before the launch. Those that fit but for the push's lists (540,000 to
+// 617,000 vertices) do so where they are few, and else run in a launch of their
+// own whose pushes walk the bitmap, a warp per row.
 #include <algorithm>
 #include <cstring>
 #include <mutex>
@@ -56,17 +59,23 @@ struct WlItem {
 };
 
 constexpr int kPullWords = 2;  // words a warp pulls at a time
+constexpr int kLeanShare = 7;  // see alb_worklist_run_device
 
-struct WlShared {
+struct WlState {
     int item, dir;
     unsigned next_word;
     unsigned n, mo, mi;  // what the level found
     int nlong;           // long rows left after their head
-    int hit;
-    PushLists rows;      // list: those long rows' numbers
 };
+// kLean: for graphs whose bitmaps leave no room for the push's lists
+template <bool kLean>
+struct WlShared : WlState {
+    PushLists rows;  // list: those long rows' numbers
+};
+template <>
+struct WlShared<true> : WlState {};
 
-__device__ __forceinline__ void wl_count(WlShared &s, unsigned n, unsigned mo, unsigned mi) {
+__device__ __forceinline__ void wl_count(WlState &s, unsigned n, unsigned mo, unsigned mi) {
     n = __reduce_add_sync(kFull, n);
     mo = __reduce_add_sync(kFull, mo);
     mi = __reduce_add_sync(kFull, mi);
@@ -94,9 +103,10 @@ __device__ __forceinline__ bool wl_scan(const WlGraph &g, const uint32_t *F, int
 }
 
 // Unvisited long rows: a warp over the first kLongChunk sources of each, the
-// CTA together over the rest of a row without a source in the frontier there.
-template <int kT>
-__device__ void wl_pull_long(const WlGraph &g, WlShared &s, const uint32_t *F, const uint32_t *V,
+// CTA together over the rest of a row without a source in the frontier there
+// (kLean: the warp over all of it).
+template <int kT, bool kLean>
+__device__ void wl_pull_long(const WlGraph &g, WlShared<kLean> &s, const uint32_t *F, const uint32_t *V,
                              uint32_t *N, int32_t *lv, int L) {
     const int lane = lane_id(), wib = threadIdx.x >> 5;
     if (threadIdx.x == 0) s.nlong = 0;
@@ -113,37 +123,41 @@ __device__ void wl_pull_long(const WlGraph &g, WlShared &s, const uint32_t *F, c
         const int32_t p = __ldg(g.lrow + i);
         if ((V[p >> 5] >> (p & 31)) & 1u) continue;
         const int64_t st = __ldg(g.lptr + i), en = __ldg(g.lptr + i + 1);
-        int64_t head = min(en, st + kLongChunk);
-        int q = 0;
+        const int64_t head = kLean ? en : min(en, st + kLongChunk);
         bool found = wl_scan(g, F, st, head);
-        if (!found && head < en) {
-            if (lane == 0) q = atomicAdd(&s.nlong, 1);
-            q = __shfl_sync(kFull, q, 0);
-            if (q < kPushRows) {
-                if (lane == 0) s.rows.list[q] = (int32_t)i;
-            } else {  // (a full list: the warp scans the whole row)
-                found = wl_scan(g, F, head, en);
+        if constexpr (!kLean) {
+            int q = 0;
+            if (!found && head < en) {
+                if (lane == 0) q = atomicAdd(&s.nlong, 1);
+                q = __shfl_sync(kFull, q, 0);
+                if (q < kPushRows) {
+                    if (lane == 0) s.rows.list[q] = (int32_t)i;
+                } else {  // (a full list: the warp scans the whole row)
+                    found = wl_scan(g, F, head, en);
+                }
             }
         }
         if (found && lane == 0) reach(p);
     }
-    __syncthreads();
-    const int left = min(s.nlong, kPushRows);
-    for (int q = 0; q < left; q++) {
-        const int32_t i = s.rows.list[q];
-        const int64_t st = __ldg(g.lptr + i) + kLongChunk, en = __ldg(g.lptr + i + 1);
-        bool found = false;
-        for (int64_t e0 = st; e0 < en && !found; e0 += (kT / 32) * kLongChunk) {
-            const int64_t b = e0 + wib * kLongChunk;
-            found = __syncthreads_or(b < en && wl_scan(g, F, b, min(en, b + kLongChunk)));
+    if constexpr (!kLean) {
+        __syncthreads();
+        const int left = min(s.nlong, kPushRows);
+        for (int q = 0; q < left; q++) {
+            const int32_t i = s.rows.list[q];
+            const int64_t st = __ldg(g.lptr + i) + kLongChunk, en = __ldg(g.lptr + i + 1);
+            bool found = false;
+            for (int64_t e0 = st; e0 < en && !found; e0 += (kT / 32) * kLongChunk) {
+                const int64_t b = e0 + wib * kLongChunk;
+                found = __syncthreads_or(b < en && wl_scan(g, F, b, min(en, b + kLongChunk)));
+            }
+            if (found && threadIdx.x == 0) reach(__ldg(g.lrow + i));
         }
-        if (found && threadIdx.x == 0) reach(__ldg(g.lrow + i));
     }
     wl_count(s, n, mo, mi);
 }
 
 // Bottom-up pull, kPullWords words per warp at a time, lane per row.
-__device__ __forceinline__ void wl_pull(const WlGraph &g, WlShared &s, const uint32_t *F,
+__device__ __forceinline__ void wl_pull(const WlGraph &g, WlState &s, const uint32_t *F,
                                         const uint32_t *V, uint32_t *N, int32_t *lv, int L) {
     const int lane = lane_id(), nw = (int)g.nwords;
     unsigned n = 0, mo = 0, mi = 0;
@@ -209,14 +223,41 @@ __device__ __forceinline__ void wl_pull(const WlGraph &g, WlShared &s, const uin
     wl_count(s, n, mo, mi);
 }
 
+// Top-down push without lists: a warp looks through 32 words at a time, lane per
+// word, and takes their rows one by one, lane per edge.
+template <class Push>
+__device__ __forceinline__ void wl_push_lean(const WlGraph &g, const uint32_t *F, int nw, int warps,
+                                             Push push) {
+    const int lane = lane_id();
+    for (int wb = (int)(threadIdx.x & ~31u); wb < nw; wb += 32 * warps) {
+        const uint32_t m = wb + lane < nw ? F[wb + lane] : 0u;
+        for (unsigned todo = __ballot_sync(kFull, m != 0); todo; todo &= todo - 1) {
+            const int q = __ffs(todo) - 1;
+            // the word's rows: their bounds by one lane each
+            const uint32_t mq = __shfl_sync(kFull, m, q);
+            int32_t st = 0, d = 0;
+            if ((mq >> lane) & 1u) {
+                const int32_t u = (wb + q) * 32 + lane;
+                st = (int32_t)__ldg(g.prow + u);
+                d = (int32_t)__ldg(g.prow + u + 1) - st;
+            }
+            for (unsigned rows = mq; rows; rows &= rows - 1) {
+                const int r = __ffs(rows) - 1;
+                const int32_t b = __shfl_sync(kFull, st, r), n = __shfl_sync(kFull, d, r);
+                for (int32_t e = lane; e < n; e += 32) push(__ldg(g.pcol + b + e));
+            }
+        }
+    }
+}
+
 // kT threads, 1024 / kT CTAs per SM.
-template <int kT>
+template <int kT, bool kLean>
 __global__ void __launch_bounds__(kT, 1024 / kT)
     k_worklist(const WlGraph *graphs, const WlItem *items, int32_t nitems, unsigned int *next_item,
                int32_t *out) {
     extern __shared__ __align__(16) unsigned char smem[];
-    WlShared &s = *reinterpret_cast<WlShared *>(smem);
-    uint32_t *maps = reinterpret_cast<uint32_t *>(smem + sizeof(WlShared));
+    WlShared<kLean> &s = *reinterpret_cast<WlShared<kLean> *>(smem);
+    uint32_t *maps = reinterpret_cast<uint32_t *>(smem + sizeof(WlShared<kLean>));
     const int lane = lane_id();
     while (true) {
         if (threadIdx.x == 0) s.item = (int)atomicAdd(next_item, 1u);
@@ -264,31 +305,36 @@ __global__ void __launch_bounds__(kT, 1024 / kT)
                 wl_pull(g, s, F, V, N, lv, L);
                 __syncthreads();
                 if (g.nlong) {
-                    wl_pull_long<kT>(g, s, F, V, N, lv, L);
+                    wl_pull_long<kT, kLean>(g, s, F, V, N, lv, L);
                     __syncthreads();
                 }
                 for (int w = threadIdx.x; w < nw; w += kT) V[w] |= N[w];
             } else {
                 for (int w = threadIdx.x; w < nw; w += kT) N[w] = 0;
-                // a frontier that fits the list is listed at once: a look at 64
-                // words at a time costs 0.3 us where they are empty and 2 where
-                // not, 60 us for 72 rows of 2^16
-                block_push<kT>(
-                    s.rows, F, 0, nw, nf <= (unsigned)kPushRows ? nw : kPushWords, g.pcol,
-                    [&](int32_t u, int32_t &st, int32_t &d, int32_t &ou) {
-                        st = (int32_t)__ldg(g.prow + u);
-                        d = (int32_t)__ldg(g.prow + u + 1) - st;
-                        ou = 0;
-                    },
-                    [&](const int32_t (&v)[4], const uint32_t (&)[4]) {
+                auto push = [&](int32_t v) {
+                    const uint32_t bit = 1u << (v & 31);
+                    if (!((V[v >> 5] | N[v >> 5]) & bit)) atomicOr(&N[v >> 5], bit);
+                };
+                if constexpr (kLean) {
+                    __syncthreads();  // (all of N is cleared)
+                    wl_push_lean(g, F, nw, kT / 32, push);
+                } else {
+                    // a frontier that fits the list is listed at once: a look at
+                    // 64 words at a time costs 0.3 us where they are empty and 2
+                    // where not, 60 us for 72 rows of 2^16
+                    block_push<kT>(
+                        s.rows, F, 0, nw, nf <= (unsigned)kPushRows ? nw : kPushWords, g.pcol,
+                        [&](int32_t u, int32_t &st, int32_t &d, int32_t &ou) {
+                            st = (int32_t)__ldg(g.prow + u);
+                            d = (int32_t)__ldg(g.prow + u + 1) - st;
+                            ou = 0;
+                        },
+                        [&](const int32_t (&v)[4], const uint32_t (&)[4]) {
 #pragma unroll
-                        for (int k = 0; k < 4; k++) {
-                            if (v[k] < 0) continue;
-                            const uint32_t bit = 1u << (v[k] & 31);
-                            if ((V[v[k] >> 5] | N[v[k] >> 5]) & bit) continue;
-                            atomicOr(&N[v[k] >> 5], bit);
-                        }
-                    });
+                            for (int k = 0; k < 4; k++)
+                                if (v[k] >= 0) push(v[k]);
+                        });
+                }
                 __syncthreads();
                 // the new frontier: levels, visited bits, counters; a warp per
                 // 32 words, lane per row
@@ -424,21 +470,38 @@ alb_status alb_worklist_run_device(alb_worklist *w, int32_t block, int32_t *d_le
     ALB_CK(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, g0->device));
     // a graph fits the kernel when its three bitmaps and the rest of the
     // shared state fit in one CTA (and its edges in 32-bit counters)
-    auto fits = [&](const Sell &s) {
-        return sizeof(uint32_t) * 3 * (size_t)s.nwords + sizeof(WlShared) + 1024 <= (size_t)max_smem &&
-               s.m_in <= INT32_MAX && s.m_out <= INT32_MAX;
+    auto fits = [&](const Sell &s, size_t state) {
+        return sizeof(uint32_t) * 3 * (size_t)s.nwords + std::max<size_t>(state, 1024) <=
+                   (size_t)max_smem && s.m_in <= INT32_MAX && s.m_out <= INT32_MAX;
     };
+    // Where there is no room for the push's lists, an item takes 13 to 25 times
+    // as long in the kernel as on the single-root path, one CTA against all SMs,
+    // but as many as there are SMs run side by side: the kernel takes them from
+    // a seventh of that on (kLeanShare). Uniform random, 580,000 vertices of mean
+    // degree 6, 16 items 2.37 ms in the kernel and 2.19 one by one, 32 2.45 and
+    // 4.30, 152 2.66 and 20.3; 560,000 of degree 40 3.23 and 1.89, 3.16 and 3.78,
+    // 2.99 and 17.9; a grid of 577,600 21.8 and 25.5, 21.8 and 50.4, 22.7 and 244.
+    struct Part {
+        std::vector<WlItem> items;
+        std::vector<int64_t> cost;
+        int64_t nwords_max = 0;
+    } part[2];  // with the lists, without
+    int64_t lean_items = 0;
+    for (const auto &e : w->entries)
+        if (e.g->sell.built && !fits(e.g->sell, sizeof(WlShared<false>) + 1024) &&
+            fits(e.g->sell, sizeof(WlShared<true>)))
+            lean_items += (int64_t)e.roots.size();
+    const bool lean = kLeanShare * lean_items >= g0->num_sms;
     std::vector<WlGraph> hg;
-    std::vector<WlItem> hi;
-    std::vector<int64_t> cost;
-    int64_t nwords_max = 0, off = 0;
+    int64_t off = 0;
     float big_ms = 0.f;
     int64_t big_kernels = 0;
     for (size_t gi = 0; gi < w->entries.size(); gi++) {
         const auto &e = w->entries[gi];
         const Sell &s = e.g->sell;
         if (!s.built) return fail(ALB_ERR_STATE, "alb_worklist_run: a graph lost its SELL build");
-        if (!fits(s)) {
+        const bool lists = fits(s, sizeof(WlShared<false>) + 1024);
+        if (!lists && !(lean && fits(s, sizeof(WlShared<true>)))) {
             // too large for one CTA's shared memory: the single-root path
             alb_bfs_opts o;
             alb_bfs_opts_default(&o);
@@ -479,15 +542,16 @@ alb_status alb_worklist_run_device(alb_worklist *w, int32_t block, int32_t *d_le
         d.alpha = e.alpha;
         d.beta = e.beta;
         hg.push_back(d);
-        nwords_max = std::max(nwords_max, s.nwords);
+        Part &p = part[lists ? 0 : 1];
+        p.nwords_max = std::max(p.nwords_max, s.nwords);
         // the kernel's graph index is the position in hg
         for (int32_t r : e.roots) {
-            hi.push_back({(int32_t)hg.size() - 1, r, off});
-            cost.push_back(e.g->nnz_in);
+            p.items.push_back({(int32_t)hg.size() - 1, r, off});
+            p.cost.push_back(e.g->nnz_in);
             off += e.g->n;
         }
     }
-    if (hi.empty()) {  // every graph took the single-root path
+    if (hg.empty()) {  // every graph took the single-root path
         if (st) {
             std::memset(st, 0, sizeof(*st));
             st->ms = big_ms;
@@ -495,18 +559,19 @@ alb_status alb_worklist_run_device(alb_worklist *w, int32_t block, int32_t *d_le
         }
         return ALB_OK;
     }
-    const size_t smem = sizeof(WlShared) + sizeof(uint32_t) * 3 * (size_t)nwords_max;
     // longest items first
-    std::vector<int32_t> order(hi.size());
-    std::iota(order.begin(), order.end(), 0);
-    std::stable_sort(order.begin(), order.end(),
-                     [&](int32_t a, int32_t b) { return cost[a] > cost[b]; });
-    std::vector<WlItem> sorted(hi.size());
-    for (size_t i = 0; i < order.size(); i++) sorted[i] = hi[order[i]];
+    std::vector<WlItem> sorted;
+    for (const Part &p : part) {
+        std::vector<int32_t> order(p.items.size());
+        std::iota(order.begin(), order.end(), 0);
+        std::stable_sort(order.begin(), order.end(),
+                         [&](int32_t a, int32_t b) { return p.cost[a] > p.cost[b]; });
+        for (int32_t k : order) sorted.push_back(p.items[k]);
+    }
     const size_t items_at = sizeof(WlGraph) * hg.size();
     const size_t ctr_at = items_at + sizeof(WlItem) * sorted.size();
     static_assert(sizeof(WlGraph) % 8 == 0 && sizeof(WlItem) % 8 == 0, "laid out one after the other");
-    const size_t args = ctr_at + 8;
+    const size_t args = ctr_at + 8;  // a counter for each part
     std::lock_guard<std::mutex> lock(w->mu);
     alb_status rc = [&]() -> alb_status {
         ALB_TRY(w->reserve(args, g0->device));
@@ -518,24 +583,39 @@ alb_status alb_worklist_run_device(alb_worklist *w, int32_t block, int32_t *d_le
         unsigned int *dctr = reinterpret_cast<unsigned int *>(w->d_args + ctr_at);
         cudaStream_t stream = g0->stream;
         ALB_CK(cudaMemcpyAsync(w->d_args, w->h_args, args, cudaMemcpyHostToDevice, stream));
-        // 1024 threads end the longest items soonest; where there are many
-        // items for every SM, two CTAs of 512 get more of them done; graphs of
-        // a word per warp of 256 threads and fewer than four have no use for more
-        const int threads = nwords_max <= 32 && block <= 256 ? 256
-                            : block == 1024 || (int64_t)sorted.size() <= 4 * (int64_t)g0->num_sms
-                                ? 1024
-                                : 512;
-        void (*f)(const WlGraph *, const WlItem *, int32_t, unsigned int *, int32_t *) =
-            threads == 256 ? k_worklist<256> : threads == 512 ? k_worklist<512> : k_worklist<1024>;
-        ALB_CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        int per_sm = 0;
-        ALB_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, threads, smem));
-        if (per_sm < 1) return fail(ALB_ERR_UNSUPPORTED, "alb_worklist_run: kernel does not fit");
-        const unsigned grid = (unsigned)std::min<int64_t>((int64_t)per_sm * g0->num_sms,
-                                                          (int64_t)sorted.size());
         ALB_CK(cudaEventRecord(g0->ev0, stream));
-        f<<<grid, threads, smem, stream>>>(dg, di, (int32_t)sorted.size(), dctr, d_levels);
-        ALB_CK(cudaGetLastError());
+        int64_t launches = 0;
+        for (int k = 0; k < 2; k++) {
+            const int64_t count = (int64_t)part[k].items.size();
+            if (count == 0) continue;
+            const int64_t nw = part[k].nwords_max;
+            // 1024 threads end the longest items soonest; where there are many
+            // items for every SM, two CTAs of 512 get more of them done; graphs
+            // of a word per warp of 256 threads and fewer than four have no use
+            // for more
+            const int threads = k == 1                      ? 1024
+                                : nw <= 32 && block <= 256 ? 256
+                                : block == 1024 || count <= 4 * (int64_t)g0->num_sms ? 1024
+                                                                                     : 512;
+            void (*f)(const WlGraph *, const WlItem *, int32_t, unsigned int *, int32_t *) =
+                k == 1           ? k_worklist<1024, true>
+                : threads == 256 ? k_worklist<256, false>
+                : threads == 512 ? k_worklist<512, false>
+                                 : k_worklist<1024, false>;
+            const size_t smem = (k ? sizeof(WlShared<true>) : sizeof(WlShared<false>)) +
+                                sizeof(uint32_t) * 3 * (size_t)nw;
+            ALB_CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            int per_sm = 0;
+            ALB_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, threads, smem));
+            if (per_sm < 1)
+                return fail(ALB_ERR_UNSUPPORTED, "alb_worklist_run: kernel does not fit");
+            const unsigned grid =
+                (unsigned)std::min<int64_t>((int64_t)per_sm * g0->num_sms, count);
+            f<<<grid, threads, smem, stream>>>(dg, di, (int32_t)count, dctr + k, d_levels);
+            ALB_CK(cudaGetLastError());
+            di += count;
+            launches++;
+        }
         ALB_CK(cudaEventRecord(g0->ev1, stream));
         ALB_CK(cudaStreamSynchronize(stream));
         float ms = 0;
@@ -543,7 +623,7 @@ alb_status alb_worklist_run_device(alb_worklist *w, int32_t block, int32_t *d_le
         if (st) {
             std::memset(st, 0, sizeof(*st));
             st->ms = ms + big_ms;
-            st->kernels = 1 + big_kernels;
+            st->kernels = launches + big_kernels;
         }
         return ALB_OK;
     }();

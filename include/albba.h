@@ -277,7 +277,8 @@ alb_status alb_msbfs64_device(alb_graph *g, const int32_t *roots, int32_t nroots
  * counter (longest graphs first). Graphs keep their own SELL build (C, sigma,
  * long rows) and Beamer thresholds. Levels only (no parents). A graph added
  * to a work list must outlive the list's runs. A graph whose bitmaps exceed
- * one CTA's shared memory (3 bits per vertex: above about 540K vertices)
+ * one CTA's shared memory (3 bits per vertex: above about 617K vertices), or
+ * leave no room beside them (above about 540K) in a list with few such items,
  * runs its items one by one on the single-root path (alb_bfs_device, the
  * entry's alpha and beta) into the same output. */
 typedef struct alb_worklist alb_worklist;
@@ -292,7 +293,8 @@ alb_status alb_worklist_size(const alb_worklist *w, int64_t *level_entries, int3
  * block: 128, 256, 512 or 1024, the least threads per CTA (the kernel takes
  * more for larger graphs). stats.ms = kernel time
  * plus the single-root runs of graphs too large for the kernel; stats.kernels
- * counts the kernel and those runs' launches. */
+ * counts the kernel's launches (a second for graphs of 540K vertices and more)
+ * and those runs'. */
 alb_status alb_worklist_run(alb_worklist *w, int32_t block, int32_t *levels, alb_stats *st);
 alb_status alb_worklist_run_device(alb_worklist *w, int32_t block, int32_t *d_levels,
                                    alb_stats *st);
