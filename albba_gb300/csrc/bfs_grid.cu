@@ -1422,6 +1422,8 @@ __global__ void __launch_bounds__(kScatterThreads)
     }
 }
 
+constexpr int kTileMax = 16384;  // the largest sort window
+
 size_t shared_bytes(int64_t nwords) {
     const int64_t stage = nwords * 4 <= kStageMax ? (nwords * 4 + 15) & ~15ll : 0;
     return kPoolAt + std::max(sizeof(Pool), (size_t)stage);
@@ -1468,9 +1470,11 @@ alb_status scatter_launch(const alb_graph *g, const BfsArgs &a, int32_t *level, 
     const bool fits = tile % 4 == 0;
     if (!fits) return ALB_ERR_UNSUPPORTED;
     const size_t smem = 2 * sizeof(int32_t) * (size_t)tile;
+    // (always the largest tile's: the limit is the function's, and another
+    // thread's search may be about to be launched)
     if (smem > 48 * 1024)
         ALB_CK(cudaFuncSetAttribute(k_scatter_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem));
+                                    (int)(2 * sizeof(int32_t) * kTileMax)));
     const int64_t tiles = (a.n + tile - 1) / tile;
     const unsigned grid = (unsigned)std::min<int64_t>(tiles, (int64_t)g->num_sms * 32);
     k_scatter_tiles<<<grid, kScatterThreads, smem, st>>>(a.n, tile, a.perm, a.level_pos,

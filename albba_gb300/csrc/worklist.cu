@@ -604,7 +604,9 @@ alb_status alb_worklist_run_device(alb_worklist *w, int32_t block, int32_t *d_le
                                  : k_worklist<1024, false>;
             const size_t smem = (k ? sizeof(WlShared<true>) : sizeof(WlShared<false>)) +
                                 sizeof(uint32_t) * 3 * (size_t)nw;
-            ALB_CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            // (always the most: the limit is the function's, and another
+            // thread's list may be about to be launched)
+            ALB_CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
             int per_sm = 0;
             ALB_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, threads, smem));
             if (per_sm < 1)
