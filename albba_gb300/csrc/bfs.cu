@@ -1867,9 +1867,10 @@ alb_status bfs_impl(alb_graph *g, int32_t root, const alb_bfs_opts &o, int32_t *
         ALB_CK(cudaGetLastError());
     }
     // the bitmaps' L2 window applies to the level loop's launches on the
-    // stream (the CUDA-graph loop carries it on its kernel nodes); it is
-    // removed again before the stream is handed back
-    const bool win = g->bfs.win.num_bytes > 0 && (coop || o.loop != ALB_LOOP_GRAPH);
+    // stream (the CUDA-graph loop carries it on its kernel nodes, the
+    // cooperative kernel on its launch); it is removed again before the stream
+    // is handed back
+    const bool win = g->bfs.win.num_bytes > 0 && !coop && o.loop != ALB_LOOP_GRAPH;
     if (win) {
         cudaStreamAttrValue v = {};
         v.accessPolicyWindow = g->bfs.win;

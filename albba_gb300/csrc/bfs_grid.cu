@@ -1447,12 +1447,21 @@ alb_status grid_launch(const alb_graph *g, const BfsArgs &a, const InitParams &i
                                                        : k_bfs_grid<false, false>;
     ALB_CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)shared_bytes(kStageMax / 4)));
-    BfsArgs aa = a;
-    InitParams ii = in;
-    GridArgs xx = x;
-    void *args[] = {&aa, &ii, &xx};
-    ALB_CK(cudaLaunchCooperativeKernel((void *)f, dim3((unsigned)g->num_sms),
-                                       dim3(kThreads), args, smem, st));
+    // the bitmaps' L2 window goes with the launch: the stream may be the
+    // caller's, and have one of its own
+    cudaLaunchAttribute at[2] = {};
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    at[1].id = cudaLaunchAttributeAccessPolicyWindow;
+    at[1].val.accessPolicyWindow = g->bfs.win;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)g->num_sms);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = g->bfs.win.num_bytes > 0 ? 2 : 1;
+    ALB_CK(cudaLaunchKernelEx(&cfg, f, a, in, x));
     return ALB_OK;
 }
 
