@@ -5,6 +5,8 @@ records nor the barrier counter's zero, whose kernel and memset were captured
 and have not run."""
 from __future__ import annotations
 
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -14,20 +16,24 @@ import oracle
 pytestmark = pytest.mark.gpu
 
 
+RELAXED = 2  # (CU_STREAM_CAPTURE_MODE_RELAXED)
+
+
 def _refused(dg, n, stream):
-    """One search while `stream` is being captured."""
+    """One search while `stream` is being captured (by the driver's API: a capture
+    of torch's that fails leaves its random numbers unusable)."""
     import torch
+    cu = C.CDLL("libcuda.so.1")
     level = torch.empty(n, dtype=torch.int32, device="cuda")
-    graph = torch.cuda.CUDAGraph()
+    h, graph = C.c_void_p(stream.cuda_stream), C.c_void_p()
     torch.cuda.synchronize()
-    with torch.cuda.stream(stream):
-        graph.capture_begin(capture_error_mode="relaxed")
-        try:
-            with pytest.raises(ab.AlbError):
-                dg.bfs_device(0, level, None)
-        finally:
-            with pytest.raises(RuntimeError):  # (the wait ended the capture)
-                graph.capture_end()
+    assert cu.cuStreamBeginCapture_v2(h, RELAXED) == 0
+    try:
+        with pytest.raises(ab.AlbError):
+            dg.bfs_device(0, level, None)
+    finally:
+        # (the wait ended the capture)
+        assert cu.cuStreamEndCapture(h, C.byref(graph)) != 0
     torch.cuda.synchronize()
 
 
