@@ -15,10 +15,11 @@
 //
 // Bound: latency. A level costs two to four dependent L2 round trips, one or
 // two cluster barriers, and the instruction fetches of code that runs once a
-// level (32-bit counters and few unrolled loops for that reason). Measured
-// against the loops of bfs.cu (CUDA graph / persistent kernel, us a call,
-// Beamer): R-MAT edge factor 16, n = 1,024: 24 (157 / 98), 65,536: 54 (198 /
-// 129); uniform random, mean degree 8, n = 65,536: 83 (326 / 203).
+// level (32-bit counters and few unrolled loops for that reason). us a call,
+// Beamer, and in brackets what the loops of bfs.cu took (CUDA graph / persistent
+// kernel): R-MAT edge factor 16, n = 1,024: 37 (180 / 118), 65,536: 70 (277 / 160);
+// uniform random, mean degree 8, n = 10,000: 51 (313 / 186), degree 3, 60,000:
+// 114 (682 / 370); grid of 65,025: 833 (6,918 / 2,403).
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -458,7 +459,8 @@ __device__ void list_level(const BfsArgs &a, Shared &s, cg::cluster_group &cl, i
     if (claimed) append(s.q[(L + 1) & 1], &s.nq[(L + 1) & 1], st, len, id);
     Counts &k = s.cnt[L & 1];
     if (kLearned) {
-        const unsigned full = __ballot_sync(kFull, word != kFull && (word | (1u << (v & 31))) == kFull);
+        const unsigned full =
+            __ballot_sync(kFull, word != kFull && (word | (1u << (v & 31))) == kFull);
         if (lane_id() == 0 && full) atomicAdd(&k.full, __popc(full));
     }
     if (!__any_sync(kFull, claimed)) return;
@@ -760,13 +762,14 @@ bool cluster_takes(const alb_graph *g, const alb_bfs_opts &o, const BfsArgs &a) 
         return false;
     // (counters are 32 bits wide)
     return g->n <= kClusterMaxN && g->sell.m_in <= INT32_MAX && g->sell.m_out <= INT32_MAX &&
-           o.loop != ALB_LOOP_HOST && !o.trace && o.policy != ALB_POLICY_BOTTOMUP_NOBYPASS && a.withhold_level < 0 && !a.short_bulk &&
-           cluster_ready(g->device);
+           o.loop != ALB_LOOP_HOST && !o.trace && o.policy != ALB_POLICY_BOTTOMUP_NOBYPASS &&
+           a.withhold_level < 0 && !a.short_bulk && cluster_ready(g->device);
 }
 
 alb_status cluster_launch(const BfsArgs &a, const InitParams &in, int32_t *d_level,
                           int32_t *d_parent, BfsCtl *result, cudaStream_t st) {
-    const Kernel f = in.policy == ALB_POLICY_LEARNED && a.mlp ? k_bfs_cluster<true> : k_bfs_cluster<false>;
+    const Kernel f = in.policy == ALB_POLICY_LEARNED && a.mlp ? k_bfs_cluster<true>
+                                                              : k_bfs_cluster<false>;
     ALB_CK(allow_cluster(f));
     cudaLaunchAttribute at;
     const cudaLaunchConfig_t cfg = config(cluster_ctas(a.nwords), map_bytes(a.nwords), st, at);

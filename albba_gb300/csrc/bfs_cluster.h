@@ -6,12 +6,15 @@
 
 namespace alb {
 
-// Largest graph (vertices) the cluster kernel takes. Against the cooperative
-// kernel on all SMs (bfs_grid.cu), us a call, Beamer / learned: R-MAT edge
-// factor 16, n = 65,536: 65 / 87 against 77 / 91, at 131,072: 87 / 135 against
-// 82 / 100; grid of 65,536: 968 / 1,447 against 1,186 / 1,793, of 131,044:
-// 1,392 / 1,617 against 1,256 / 1,240; uniform random, mean degree 8, 32,768:
-// 62 / 109 against 82 / 84, 65,536: 93 / 149 against 85 / 94.
+// Largest graph (vertices) the cluster kernel takes: where the default policy's
+// searches of R-MAT and uniform random graphs meet those of the cooperative
+// kernel on all SMs (bfs_grid.cu). us a call, cluster against cooperative,
+// Beamer; learned: R-MAT edge factor 16, n = 1,024: 37 / 63; 62 / 68, 65,536:
+// 71 / 82; 107 / 97, 131,072: 103 / 85; 110 / 87. Uniform random, mean degree 8,
+// 32,768: 66 / 86; 115 / 94, 65,536: 90 / 92; 142 / 101, 131,072: 123 / 86; 189 /
+// 118. Grids of 65,536: 861 / 1,097; 1,300 / 1,585, of 131,044: 1,258 / 1,404; 1,393
+// / 1,563. The learned policy pushes more, and so crosses at fewer vertices;
+// where there are many edges a vertex it is sent away (cluster_takes).
 constexpr int64_t kClusterMaxN = 1 << 16;
 
 // Whether the call runs as one cluster launch. Calls that ask for what only

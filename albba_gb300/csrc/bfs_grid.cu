@@ -1,8 +1,8 @@
 // Single-root BFS as one cooperative kernel, one block of 1024 threads per SM:
 // initial state, every level, counters. Outputs are written by a second kernel
 // (k_scatter_tiles). It serves both device-driven loops of graphs too large
-// for one cluster (bfs_cluster.cu); traced runs and the pull without bypass
-// keep the kernels of bfs.cu, whose counters they report.
+// for one cluster, or too dense for its pushes (bfs_cluster.cu); traced runs and
+// the pull without bypass keep the kernels of bfs.cu, whose counters they report.
 //
 // Blocks meet at one arrival counter (1.3 us; records that every block stores
 // and every block polls took 4.6, on lines of their own 2.2). What a phase

@@ -192,12 +192,13 @@ __device__ __forceinline__ void ms_start(const MsArgs &a, const MsInit &in, int6
 // Words of a bottom-up level in runs of `run` words (1 to 32, set by the
 // host from the word count: about three runs per warp) from the level's
 // counter (dynamic distribution, as WordRuns); where x.numbered is set a warp's
-// first run goes by its number, which saves a round trip. The done words of a run are loaded together, one per lane, a run
-// ahead of use. kSkip: words whose rows are all done are not yielded; their
-// next-frontier words and nonzero bits are cleared when the run comes up, one
-// coalesced store per word, so a warp does not walk them one dependent round
-// trip at a time (at late levels most words are such). Words of slices wider
-// than `split` are left to ms_pull_wide. Call from all lanes of a warp.
+// first run goes by its number, which saves a round trip. The done words of a
+// run are loaded together, one per lane, a run ahead of use. kSkip: words whose
+// rows are all done are not yielded; their next-frontier words and nonzero bits
+// are cleared when the run comes up, one coalesced store per word, so a warp
+// does not walk them one dependent round trip at a time (at late levels most
+// words are such). Words of slices wider than `split` are left to ms_pull_wide.
+// Call from all lanes of a warp.
 template <bool kSkip>
 struct MsWords {
     int32_t cur, nxt;     // first word of the current run and of the next one

@@ -6,10 +6,10 @@
 // to 10 kernels behind a switch and a while node, about 43 us on R-MAT scale
 // 16 whatever the level held. Here a level takes one barrier (a pull) to five
 // (a push with long rows and samples), some 1.5 us each, and steps without
-// work are not run. 37 roots on R-MAT scale 16, search and output: 418 -> 175
-// us; 64 on scale 20: 690 -> 409; 64 on scale 24: 3,565 -> 3,340, of which the
-// two large pulls (970 and 400) are bound by their gathers, one address per
-// clock and SM, and the output (870) by memory.
+// work are not run. 37 roots on R-MAT scale 16, a call with its output: 420 ->
+// 153 us; 64 on scale 20 (learned policy) 728 -> 415; 64 on scale 24 (learned,
+// random roots) 3,433 -> 3,175, of which the large pulls (870 to 970 and 240 to
+// 400) are bound by their gathers and the output (870) by memory.
 //
 // The block keeps under 8 KB of shared memory: L1 holds the gathers' hubs.
 // With 40 KB (the selector's weights and a frontier row table copied there)

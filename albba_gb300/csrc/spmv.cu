@@ -24,12 +24,14 @@
 // milliseconds. They are kept in a list of their own, longest first. The
 // chain of fused multiply-adds is what makes y bit-identical, and a dependent
 // fp64 fma costs about 115 cycles on GB300 (for one active lane as for 32), so
-// the list is summed in two ways: shorter ones lane per row (k_spmv_long: 32 chains side by side), the hubs
-// CTA per row with the chain's steps found 256 at a time as integers
-// (k_spmv_hub, chain.cuh), so that the longest row's chain no longer sets the
-// launch's length. Each runs on a stream of its own beside the slices. R-MAT
-// scale 22, edge factor 16, signed values: 9.47 ms with every long row lane
-// per row, 2.1 ms now; with positive values 0.84 ms.
+// the list is summed in two ways: most lane per row (k_spmv_long: 32 chains side
+// by side), and where a few are much longer those CTA per row with the chain's
+// steps found 256 at a time as integers (k_spmv_hub, chain.cuh; hub_rows says
+// which), so that the longest row's chain no longer sets the launch's length.
+// Each runs on a stream of its own beside the slices. R-MAT scale 22, edge factor
+// 16, signed values: 9.45 ms with every long row lane per row, 1.9 to 2.2 ms now;
+// with positive values 0.85 ms. The longest row alone takes 6.6 ns an entry, and
+// about twice that beside the others on its SM.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -546,14 +548,14 @@ __global__ void k_sp_hub_fill(int64_t nlong, const int32_t *lrow, const int64_t 
 // each. Lane per row does 32 rows at once but takes kLaneNs per entry of its
 // longest. A hub row's CTA takes 3 ns per entry and, for signed terms, 0.35 us
 // at each of the entries that leave the binade: about kHubNs per entry, and no
-// more than kHubRootNs times the root of the length, all in all. Up to two CTAs
-// an SM run as fast as one; more share the SM, and each then takes kShareNs per
-// entry and kShareRootNs per root of the time of all SMs together. Signed terms
-// are what is reckoned with: x is not known yet.
+// more than kHubRootNs times the root of the length, all in all. wave: CTAs that
+// run at once (two an SM, by their registers). Where there are more, each takes
+// kShareNs per entry and kShareRootNs per root of the time of all SMs together.
+// Signed terms are what is reckoned with: x is not known yet.
 //
 // The line between the two is drawn low, where the longest lane-per-row chain
-// ends well before the longest hub's, unless more rows than two an SM are above
-// it; then at the lowest length whose reckoned time is within a tenth of the
+// ends well before the longest hub's, unless more rows than a wave are above it;
+// then at the lowest length whose reckoned time is within a tenth of the
 // best. us, signed / positive terms: 100,000 rows of 1,000 entries take 418 lane
 // per row and 15,199 / 3,926 as hubs, 900 of 4,000 241 and 517 / 80, 600 of 30,000
 // 1,950 and 1,516 / 300, 150 of 1,000 59 and 81 / 20; R-MAT scale 22 (longest row
@@ -561,13 +563,13 @@ __global__ void k_sp_hub_fill(int64_t nlong, const int32_t *lrow, const int64_t 
 // 1.25 at 6, scale 16 (10,000) 0.34 / 0.07, 0.34 / 0.12 and 0.34 / 0.06.
 constexpr double kLaneNs = 58, kHubNs = 80, kHubRootNs = 4400, kShareNs = 0.032, kShareRootNs = 4.8;
 
-int64_t hub_rows(const std::vector<int32_t> &len, int num_sms) {
+int64_t hub_rows(const std::vector<int32_t> &len, int64_t wave) {
     auto above = [&](double t) -> int64_t {  // rows longer than t
         return std::lower_bound(len.begin(), len.end(), (int32_t)t, std::greater<int32_t>()) -
                len.begin();
     };
     const double longest = len[0], low = std::max((double)kSpLong, 12.0 * std::sqrt(longest));
-    if (above(low) <= 2 * (int64_t)num_sms) return above(low);
+    if (above(low) <= wave) return above(low);
     auto alone = [](double n) { return std::min(kHubNs * n, kHubRootNs * std::sqrt(n)); };
     std::vector<double> all(1, 0.0);  // all[k]: what the first k rows take of all SMs
     for (int64_t i = 0; i < above(low); i++)
@@ -577,7 +579,7 @@ int64_t hub_rows(const std::vector<int32_t> &len, int num_sms) {
         const int64_t k = above(t);
         double ns = k < (int64_t)len.size() ? kLaneNs * len[(size_t)k] : 0.0;
         if (k > 0) ns = std::max(ns, alone(longest));
-        if (k > 2 * (int64_t)num_sms) ns = std::max(ns, all[(size_t)k] + alone(len[(size_t)k - 1]) / 2);
+        if (k > wave) ns = std::max(ns, all[(size_t)k] + alone(len[(size_t)k - 1]) / 2);
         line.emplace_back(k, ns);
         if (k == 0) break;
     }
@@ -684,7 +686,9 @@ alb_status build(alb_sellmat *m, const int64_t *rowptr, const int32_t *col, cons
                 srow[(size_t)i] = hrow[(size_t)order[(size_t)i]];
                 slen[(size_t)i] = (int32_t)hlen[(size_t)order[(size_t)i]];
             }
-            m->nhub = hub_rows(slen, m->num_sms);
+            m->nhub = hub_rows(slen, (int64_t)m->num_sms *
+                                         std::max(1, resident_blocks((const void *)k_spmv_hub,
+                                                                     kHubThreads)));
             // hubs: rows one after the other, each padded to kLb entries; the
             // others: slices of 32 rows, as wide as the first (longest) one
             for (int64_t i = 0; i < m->nhub; i++)
