@@ -555,21 +555,30 @@ __global__ void k_sp_hub_fill(int64_t nlong, const int32_t *lrow, const int64_t 
 //
 // The line between the two is drawn low, where the longest lane-per-row chain
 // ends well before the longest hub's, unless more rows than a wave are above it;
-// then at the lowest length whose reckoned time is within a tenth of the
-// best. us, signed / positive terms: 100,000 rows of 1,000 entries take 418 lane
+// then at the lowest length whose reckoned time is within a tenth of the best.
+// Rows of up to kMixedMost entries are left to the lanes where their values have
+// both signs, which mostly means that the terms have (mixed(i): row i's values
+// have): 30 rows of 600 take 37 us so and 51 as hubs, of 1,000 59 and 80 (17 and 19
+// with positive terms). us, signed / positive terms: 100,000 rows of 1,000 entries take 418 lane
 // per row and 15,199 / 3,926 as hubs, 900 of 4,000 241 and 517 / 80, 600 of 30,000
 // 1,950 and 1,516 / 300, 150 of 1,000 59 and 81 / 20; R-MAT scale 22 (longest row
 // 163,186) 2.29 / 0.85 ms with the line at 12 sqrt(N), 2.22 / 0.81 at 25 and 4.10 /
 // 1.25 at 6, scale 16 (10,000) 0.34 / 0.07, 0.34 / 0.12 and 0.34 / 0.06.
 constexpr double kLaneNs = 58, kHubNs = 80, kHubRootNs = 4400, kShareNs = 0.032, kShareRootNs = 4.8;
+constexpr int32_t kMixedMost = 1000;
 
-int64_t hub_rows(const std::vector<int32_t> &len, int64_t wave) {
+template <class Mixed>
+int64_t hub_rows(const std::vector<int32_t> &len, int64_t wave, Mixed mixed) {
     auto above = [&](double t) -> int64_t {  // rows longer than t
         return std::lower_bound(len.begin(), len.end(), (int32_t)t, std::greater<int32_t>()) -
                len.begin();
     };
     const double longest = len[0], low = std::max((double)kSpLong, 12.0 * std::sqrt(longest));
-    if (above(low) <= wave) return above(low);
+    if (above(low) <= wave) {
+        for (int64_t i = above(kMixedMost); i < above(low); i++)
+            if (mixed(i)) return above(std::max(low, (double)kMixedMost));
+        return above(low);
+    }
     auto alone = [](double n) { return std::min(kHubNs * n, kHubRootNs * std::sqrt(n)); };
     std::vector<double> all(1, 0.0);  // all[k]: what the first k rows take of all SMs
     for (int64_t i = 0; i < above(low); i++)
@@ -686,9 +695,13 @@ alb_status build(alb_sellmat *m, const int64_t *rowptr, const int32_t *col, cons
                 srow[(size_t)i] = hrow[(size_t)order[(size_t)i]];
                 slen[(size_t)i] = (int32_t)hlen[(size_t)order[(size_t)i]];
             }
-            m->nhub = hub_rows(slen, (int64_t)m->num_sms *
-                                         std::max(1, resident_blocks((const void *)k_spmv_hub,
-                                                                     kHubThreads)));
+            auto mixed = [&](int64_t i) {
+                const double *b = val + rowptr[srow[(size_t)i]], *e = b + slen[(size_t)i];
+                return std::any_of(b, e, [](double v) { return v > 0; }) &&
+                       std::any_of(b, e, [](double v) { return v < 0; });
+            };
+            const int per = resident_blocks((const void *)k_spmv_hub, kHubThreads);
+            m->nhub = hub_rows(slen, (int64_t)m->num_sms * std::max(1, per), mixed);
             // hubs: rows one after the other, each padded to kLb entries; the
             // others: slices of 32 rows, as wide as the first (longest) one
             for (int64_t i = 0; i < m->nhub; i++)

@@ -14,21 +14,22 @@ import oracle
 pytestmark = pytest.mark.gpu
 
 
-def _matrix(rows, length, rng):
+def _matrix(rows, length, rng, low=-1):
     lens = np.full(rows, length) + rng.integers(0, 9, rows)
     n = max(rows, 2 * length)
     rp = np.zeros(n + 1, np.int64)
     rp[1:rows + 1] = np.cumsum(lens)
     rp[rows + 1:] = rp[rows]
-    return rp, rng.integers(0, n, rp[-1]).astype(np.int32), rng.uniform(-1, 1, rp[-1])
+    return rp, rng.integers(0, n, rp[-1]).astype(np.int32), rng.uniform(low, 1, rp[-1])
 
 
-# two CTAs an SM, just over, more than a wave of six an SM
-@pytest.mark.parametrize("rows,length", [(300, 300), (304, 700), (305, 700), (305, 5000),
-                                         (1000, 260), (3000, 900), (40, 9000)])
-def test_bit_exact(rows, length):
+# two CTAs an SM, just over, many more; up to 1,000 entries a row's signs count
+@pytest.mark.parametrize("low", [-1, 0])
+@pytest.mark.parametrize("rows,length", [(300, 300), (304, 700), (305, 700), (305, 5000), (40, 992),
+                                         (40, 993), (1000, 260), (3000, 900), (40, 9000)])
+def test_bit_exact(rows, length, low):
     rng = np.random.default_rng(rows)
-    rp, col, val = _matrix(rows, length, rng)
+    rp, col, val = _matrix(rows, length, rng, low)
     x = rng.standard_normal(len(rp) - 1)
     with ab.SellMatrix(rp, col, val) as m:
         assert np.array_equal(m.spmv(x).view(np.uint64), oracle.spmv(rp, col, val, x).view(np.uint64))
